@@ -125,8 +125,12 @@ struct Impl : ImplBase {
     int n = 0;
     int64_t* ptr = nullptr;
     int* idx = nullptr;
-    int64_t* ptr2 = nullptr;
     int* idx2 = nullptr;
+    // leaf pass: items, cut rounds and their partial sums
+    LeafItem* items = nullptr;
+    LeafSplit* splits = nullptr;
+    int nitem = 0, nsplit = 0;
+    void* partial = nullptr;
     // GEMM column lists over R density vectors: the node lists repeated
     // with offsets r * nnodes into the [r][node][...] buffers (aux offset
     // too when it holds node ids, copied when it holds levels)
@@ -289,7 +293,6 @@ struct Impl : ImplBase {
       a64.tx = upload(tl[0]);
       a64.ty = upload(tl[1]);
       a64.tz = upload(tl[2]);
-      a64.l2t_depth = 1 << 30;  // near field only
     }
     // ---- surfaces and operators
     args.ue_unit = upload_as_T(op.ue);
@@ -498,8 +501,13 @@ struct Impl : ImplBase {
         mptr.push_back((int64_t)midx.size());
       }
       s2l = make_list(xw, {}, xptr, xidx);
-      leaf = make_list(lw, {}, nptr, nidx, mptr, midx);
-      if (near64) near_u = make_list(lw, {}, uptr, uidx, std::vector<int64_t>(lw.size() + 1, 0), {});
+      std::vector<unsigned char> l2t(lw.size());
+      for (size_t k = 0; k < lw.size(); k++) l2t[k] = tr.depth[lw[k]] >= 2;
+      leaf = make_leaf_list<T>(lw, nptr, nidx, mptr, midx, l2t, td_u);
+      // the FP64 near field of a double layer beside the FP32 passes: points only
+      if (near64)
+        near_u = make_leaf_list<double>(lw, uptr, uidx, std::vector<int64_t>(lw.size() + 1, 0), {},
+                                        std::vector<unsigned char>(lw.size(), 0), td_u);
       for (int g : v_s2m) surf_int += (double)nuc * tr.scnt[g];
       counters_near = near_int;
       counters_surf = surf_int;
@@ -781,8 +789,7 @@ struct Impl : ImplBase {
          counters_gemm = 0, counters_tc_had = 0;
 
   List make_list(const std::vector<int>& work, const std::vector<int>& aux, const std::vector<int64_t>& ptr = {},
-                 const std::vector<int>& idx = {}, const std::vector<int64_t>& ptr2 = {},
-                 const std::vector<int>& idx2 = {}) {
+                 const std::vector<int>& idx = {}) {
     List l;
     l.n = (int)work.size();
     l.work = upload(work);
@@ -791,11 +798,46 @@ struct Impl : ImplBase {
       l.ptr = upload(ptr);
       l.idx = upload(idx);
     }
-    if (!ptr2.empty()) {
-      l.ptr2 = upload(ptr2);
-      l.idx2 = upload(idx2);
+    return l;
+  }
+
+  // the leaf pass over leaves `lw` in precision U
+  template <class U>
+  List make_leaf_list(const std::vector<int>& lw, const std::vector<int64_t>& nptr, const std::vector<int>& nidx,
+                      const std::vector<int64_t>& mptr, const std::vector<int>& midx,
+                      const std::vector<unsigned char>& l2t, int td) {
+    List l;
+    l.n = (int)lw.size();
+    l.idx = upload(nidx);
+    l.idx2 = upload(midx);
+    std::vector<LeafItem> items;
+    std::vector<LeafSplit> splits;
+    int nparts = 0;
+    leaf_items(l.n, lw.data(), tr.tcnt.data(), tr.scnt.data(), nptr.data(), nidx.data(), mptr.data(), l2t.data(),
+               tr.tbeg.data(), nsurf, sizeof(U) == 8 ? 128 : 256, num_sms, &items, &splits, &nparts);
+    l.nitem = (int)items.size();
+    l.nsplit = (int)splits.size();
+    l.items = upload(items);
+    if (l.nsplit > 0) {
+      l.splits = upload(splits);
+      l.partial = dalloc<U>((size_t)nparts * 32 * td);
     }
     return l;
+  }
+
+  P2PWork p2p_work(const List& l) const {
+    P2PWork w;
+    w.work = l.work;
+    w.n = l.n;
+    w.ptr = l.ptr;
+    w.idx = l.idx;
+    w.idx2 = l.idx2;
+    w.items = l.items;
+    w.nitem = l.nitem;
+    w.splits = l.splits;
+    w.nsplit = l.nsplit;
+    w.partial = l.partial;
+    return w;
   }
 
   size_t S_supe = 0, S_supc = 0, S_tdnc = 0, S_tdne = 0, S_y = 0, S_z = 0, S_spec = 0, S_eff = 0;
@@ -887,20 +929,13 @@ struct Impl : ImplBase {
   // densities and potentials) on slice r of the per-vector node data
   void p2p(const List& l, int which, int rhs, int r, cudaStream_t st) {
     if (l.n <= 0) return;
-    P2PWork w;
-    w.work = l.work;
-    w.n = l.n;
-    w.ptr = l.ptr;
-    w.idx = l.idx;
-    w.ptr2 = l.ptr2;
-    w.idx2 = l.idx2;
     P2PArgs<T> a = args;
     a.supeden = supeden + (size_t)r * S_supe;
     a.supcval = supcval + (size_t)r * S_supc;
     a.tdncval = tdncval + (size_t)r * S_tdnc;
     a.tdneden = tdneden + (size_t)r * S_tdne;
-    launch_p2p<T>(E.user.kt, a, w, which, rhs, st);
-    nlaunch++;
+    launch_p2p<T>(E.user.kt, a, p2p_work(l), which, rhs, st);
+    nlaunch += l.nsplit > 0 ? 2 : 1;
   }
 
   // the V list for density vector slice r: forward spectra, Hadamard, inverse
@@ -1039,15 +1074,8 @@ struct Impl : ImplBase {
       for (int r = 0; r < R; r++) {
         p2p(leaf, P2P_LEAF, r0 + r, r, st);
         if (near64 && near_u.n > 0) {
-          P2PWork w;
-          w.work = near_u.work;
-          w.n = near_u.n;
-          w.ptr = near_u.ptr;
-          w.idx = near_u.idx;
-          w.ptr2 = near_u.ptr2;
-          w.idx2 = near_u.idx2;
-          launch_p2p<double>(E.user.kt, a64, w, P2P_LEAF, r0 + r, st);
-          nlaunch++;
+          launch_p2p<double>(E.user.kt, a64, p2p_work(near_u), P2P_LEAF, r0 + r, st);
+          nlaunch += near_u.nsplit > 0 ? 2 : 1;
         }
       }
       if (prof) KCHECK(cudaEventRecord(ev[5], st));
@@ -1106,13 +1134,13 @@ Engine::~Engine() { release_device(); }
 
 void Engine::release_device() {
   impl.reset();
-  double** bufs[] = {&d_in, &d_out, &d_spos, &d_snor, &d_sden, &d_tchk, &d_vchk};
+  double** bufs[] = {&d_in, &d_out, &d_spos, &d_snor, &d_sden, &d_tchk, &d_vchk, &d_dpart};
   for (double** b : bufs)
     if (*b) {
       cudaFree(*b);
       *b = nullptr;
     }
-  d_in_cap = d_out_cap = d_sden_cap = d_tchk_cap = 0;
+  d_in_cap = d_out_cap = d_sden_cap = d_tchk_cap = d_dpart_cap = 0;
   if (stream) {
     cudaStreamDestroy(stream);
     stream = nullptr;
@@ -1820,9 +1848,11 @@ int Engine::direct(const double* srcden, int ntc, const double* tpos, double* ou
   try {
     if (!d_spos) {
       KCHECK(cudaMalloc(&d_spos, std::max<size_t>(1, 3 * (size_t)ns) * sizeof(double)));
+      KCHECK(cudaMemcpyAsync(d_spos, srcpos.data(), 3 * (size_t)ns * sizeof(double), cudaMemcpyHostToDevice, stream));
+    }
+    if (!d_snor && user.dl) {
       KCHECK(cudaMalloc(&d_snor, std::max<size_t>(1, 3 * (size_t)ns) * sizeof(double)));
-      KCHECK(cudaMemcpy(d_spos, srcpos.data(), 3 * (size_t)ns * sizeof(double), cudaMemcpyHostToDevice));
-      KCHECK(cudaMemcpy(d_snor, srcnor.data(), 3 * (size_t)ns * sizeof(double), cudaMemcpyHostToDevice));
+      KCHECK(cudaMemcpyAsync(d_snor, srcnor.data(), 3 * (size_t)ns * sizeof(double), cudaMemcpyHostToDevice, stream));
     }
     size_t nden = (size_t)ns * user.sd;
     if (nden > d_sden_cap || !d_sden) {
@@ -1831,7 +1861,7 @@ int Engine::direct(const double* srcden, int ntc, const double* tpos, double* ou
       KCHECK(cudaMalloc(&d_sden, std::max<size_t>(1, nden) * sizeof(double)));
       d_sden_cap = nden;
     }
-    KCHECK(cudaMemcpy(d_sden, srcden, nden * sizeof(double), cudaMemcpyHostToDevice));
+    KCHECK(cudaMemcpyAsync(d_sden, srcden, nden * sizeof(double), cudaMemcpyHostToDevice, stream));
     size_t ntp = std::max<size_t>(1, (size_t)ntc);
     if (ntp > d_tchk_cap || !d_tchk) {
       if (d_tchk) cudaFree(d_tchk);
@@ -1841,10 +1871,21 @@ int Engine::direct(const double* srcden, int ntc, const double* tpos, double* ou
       KCHECK(cudaMalloc(&d_vchk, 4 * ntp * sizeof(double)));
       d_tchk_cap = ntp;
     }
-    KCHECK(cudaMemcpy(d_tchk, tpos, 3 * (size_t)ntc * sizeof(double), cudaMemcpyHostToDevice));
+    KCHECK(cudaMemcpyAsync(d_tchk, tpos, 3 * (size_t)ntc * sizeof(double), cudaMemcpyHostToDevice, stream));
     double kc[3];
     kernel_constants(user.kt, user.coefs, kc);
-    launch_direct(user.kt, d_spos, d_snor, d_sden, ns, d_tchk, ntc, d_vchk, kc, stream);
+    int sms = 0;
+    KCHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    // (a plan's partial sums are at most 16 CTAs per SM x 128 targets x 3: 7.3 MB)
+    const DirectPlan plan = direct_plan(ns, ntc, user.td, sms, (size_t)1 << 20);
+    if (plan.scratch > d_dpart_cap) {
+      if (d_dpart) cudaFree(d_dpart);
+      d_dpart = nullptr;
+      d_dpart_cap = 0;
+      KCHECK(cudaMalloc(&d_dpart, plan.scratch * sizeof(double)));
+      d_dpart_cap = plan.scratch;
+    }
+    launch_direct(user.kt, plan, d_spos, d_snor, d_sden, ns, d_tchk, ntc, d_vchk, d_dpart, kc, sms, stream);
     KCHECK(cudaGetLastError());
     KCHECK(cudaMemcpyAsync(out, d_vchk, (size_t)ntc * user.td * sizeof(double), cudaMemcpyDeviceToHost, stream));
     KCHECK(cudaStreamSynchronize(stream));

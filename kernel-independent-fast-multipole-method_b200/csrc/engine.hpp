@@ -84,7 +84,8 @@ struct Engine {
   size_t d_in_cap = 0, d_out_cap = 0;
   // original-order copies for the direct sum (uploaded on first use)
   double *d_spos = nullptr, *d_snor = nullptr, *d_sden = nullptr, *d_tchk = nullptr, *d_vchk = nullptr;
-  size_t d_sden_cap = 0, d_tchk_cap = 0;
+  double* d_dpart = nullptr;  // partial sums of the source chunks
+  size_t d_sden_cap = 0, d_tchk_cap = 0, d_dpart_cap = 0;
 
   ~Engine();
   int setup();  // returns a kifmm_status

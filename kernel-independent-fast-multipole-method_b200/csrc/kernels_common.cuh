@@ -48,12 +48,37 @@ __device__ __forceinline__ float rsqrt_t(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt(x); }
+// FP64: the approximate reciprocal root (rsqrt.approx.ftz.f64, 9.3e-7 measured)
+// and one step of Householder's third-order iteration on it, with the residual
+// e = 1 - x y^2: y (1 + e/2 + 3 e^2 / 8), error 5 e^3 / 16 < 3e-18.  For
+// normal, finite x; within one unit in the last place of rsqrt() over
+// [1e-16, 1e2].  Five FP64 instructions and no special-case branch
+// (dependent chains of each, 148 SMs: 2.55e12 per second, rsqrt() 1.75e12);
+// the FP64 pipe (64 lanes per SM and clock) bounds every FP64 sum.
+__device__ __forceinline__ double rsqrt_t(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = __fma_rn(-(x * y), y, 1.0);
+  return __fma_rn(y * e, __fma_rn(0.375, e, 0.5), y);
+}
+
+// 1/r from r^2, 0 below the cut-off r^2 < 1e-16
+__device__ __forceinline__ float rinv_cut(float r2) { return (r2 >= 1e-16f) ? rsqrt_t(r2) : 0.f; }
+// FP64: the cut-off, an infinite and a NaN r^2 (1/r = 0, as from rsqrt() and
+// from the failed comparison) in one unsigned range test of the bit pattern,
+// which leaves the FP64 pipe to the sum
+__device__ __forceinline__ double rinv_cut(double r2) {
+  constexpr unsigned long long lo = 0x3C9CD2B297D889BCull;  // 1e-16
+  constexpr unsigned long long inf = 0x7FF0000000000000ull;
+  const bool in = (unsigned long long)__double_as_longlong(r2) - lo < inf - lo;
+  const double ri = rsqrt_t(r2);
+  return in ? ri : 0.0;
+}
 
 template <int KT, typename T>
 __device__ __forceinline__ void keval(T x, T y, T z, const T* nrm, const T* f, T* u, const KConst<T>& k) {
   T r2 = x * x + y * y + z * z;
-  T ri = (r2 >= T(1e-16)) ? rsqrt_t(r2) : T(0);
+  T ri = rinv_cut(r2);
   if constexpr (KT == 111) {  // 1/(4 pi r)
     u[0] += k.c0 * ri * f[0];
   } else if constexpr (KT == 121) {  // -(r.n)/(4 pi r^3)

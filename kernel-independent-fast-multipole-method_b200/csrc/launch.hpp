@@ -31,28 +31,59 @@ struct P2PArgs {
   T* supcval = nullptr;
   T* tdncval = nullptr;
   KConst<T> ku{}, km{};  // user and equivalent kernel constants
-  // leaves at this depth and below add L2T from their downward equivalent
-  // surface in the leaf pass (a pass with near-field sources only sets it
-  // beyond the deepest level)
-  int l2t_depth = 2;
 };
 
 enum { P2P_S2M = 0, P2P_S2L = 1, P2P_LEAF = 2 };
 
+// One warp's work in the leaf pass: targets [tb, tb + 32) of leaf g against
+// point sources (near-list segments nb .. nb + nn, from `skip` sources into the
+// first, `take` in all), W-list surfaces mb .. mb + nm and, if l2t, the leaf's own
+// downward equivalent surface; the sum goes to the leaf's potentials (out < 0)
+// or to the partial sums' row `out`.
+struct LeafItem {
+  int64_t nb = 0, mb = 0;
+  int g = 0, tb = 0, nn = 0, skip = 0, take = 0, nm = 0, l2t = 0, out = -1;
+};
+// A round of targets whose sources several items share: targets [tbeg, tbeg +
+// cnt) = the sum of the partial rows first .. first + parts.
+struct LeafSplit {
+  int tbeg, cnt, first, parts;
+};
+// host side: the items of the leaves `work` (source counts scnt, near lists
+// nptr/nidx, W-list surface counts from mptr, l2t flags per leaf), the rounds
+// that were cut and their number of partial rows
+void leaf_items(int nwork, const int* work, const int* tcnt, const int* scnt, const int64_t* nptr, const int* nidx,
+                const int64_t* mptr, const unsigned char* l2t, const int* tbeg, int nsurf, int least, int num_sms,
+                std::vector<LeafItem>* items, std::vector<LeafSplit>* splits, int* nparts);
+
 struct P2PWork {
-  const int* work = nullptr;  // node ids, one CTA each
+  const int* work = nullptr;  // node ids, one CTA each (S2M: one warp)
   int n = 0;
-  const int64_t* ptr = nullptr;  // CSR over work items (S2L: X leaves; LEAF: point-source leaves)
-  const int* idx = nullptr;
-  const int64_t* ptr2 = nullptr;  // LEAF: M2T source nodes
-  const int* idx2 = nullptr;
+  const int64_t* ptr = nullptr;  // S2L: CSR over work items, X leaves
+  const int* idx = nullptr;      // S2L: X leaves; LEAF: point-source leaves
+  const int* idx2 = nullptr;     // LEAF: M2T source nodes
+  // LEAF: the items, the cut rounds and their partial sums [row][32][td]
+  const LeafItem* items = nullptr;
+  int nitem = 0;
+  const LeafSplit* splits = nullptr;
+  int nsplit = 0;
+  void* partial = nullptr;
 };
 
 template <typename T>
 void launch_p2p(int kt, const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cudaStream_t st);
 
-void launch_direct(int kt, const double* spos, const double* snor, const double* sden, int ns, const double* tpos,
-                   int nt, double* out, const double* kc3, cudaStream_t st);
+// Direct sum (direct.cu): the split of the sources into chunks, whose partial
+// potentials take `scratch` doubles (0: one chunk, written straight to out).
+struct DirectPlan {
+  int G = 128, tblocks = 0, nchunk = 1, chunk = 1;
+  size_t scratch = 0;
+};
+DirectPlan direct_plan(int ns, int nt, int td, int num_sms, size_t capacity);
+// snor is read for double-layer kernels only
+void launch_direct(int kt, const DirectPlan& p, const double* spos, const double* snor, const double* sden, int ns,
+                   const double* tpos, int nt, double* out, double* scratch, const double* kc3, int num_sms,
+                   cudaStream_t st);
 
 template <typename T>
 void launch_scatter_den(const double* srcden, const int* perm, int ns, int sd, int nrhs, T* out, cudaStream_t st);

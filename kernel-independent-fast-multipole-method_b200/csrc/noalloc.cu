@@ -11,7 +11,7 @@
 // an entry point that allocates nothing else.
 //
 // How: the sources are split into chunks evaluated by different CTAs (so a
-// small target set still fills the GPU); each chunk's partial potentials go
+// small target set still fills the GPU, direct.cu); each chunk's partial potentials go
 // to a fixed scratch array in device global memory, declared below at file
 // scope, and a second kernel adds the chunks up into the caller's output.
 // The scratch holds KIFMM_NOALLOC_SCRATCH_DOUBLES doubles (8 MiB) on every
@@ -29,76 +29,13 @@
 // lookup allocates nothing and stays right after a cudaDeviceReset, which
 // reloads the module and may move the array.  The first call on a device
 // loads the module there and should come before any stream capture.
-#include <algorithm>
-
 #include "../../include/kifmm.h"
-#include "kernels_common.cuh"
+#include "launch.hpp"
 
 namespace kifmm {
 namespace {
 
 static __device__ __align__(256) double g_noalloc_scratch[KIFMM_NOALLOC_SCRATCH_DOUBLES];
-
-constexpr int NA_THREADS = 128;
-constexpr int NA_TILE = 128;
-constexpr int NA_MAXCHUNK = 64;
-
-// partial[c][t][d] = sum over sources of chunk c of K(trg_t - src) den
-template <int KT>
-__global__ void __launch_bounds__(NA_THREADS) k_direct_partial(const double* __restrict__ spos,
-                                                               const double* __restrict__ snor,
-                                                               const double* __restrict__ sden, int ns, int chunk,
-                                                               const double* __restrict__ tpos, int nt,
-                                                               double* __restrict__ partial, KConst<double> kc) {
-  constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD;
-  __shared__ double sx[NA_TILE], sy[NA_TILE], sz[NA_TILE], nx[NA_TILE], ny[NA_TILE], nz[NA_TILE], f[NA_TILE * 4];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s0 = blockIdx.y * chunk;
-  const int s1 = min(ns, s0 + chunk);
-  double px = 0, py = 0, pz = 0;
-  if (t < nt) {
-    px = tpos[3 * (size_t)t];
-    py = tpos[3 * (size_t)t + 1];
-    pz = tpos[3 * (size_t)t + 2];
-  }
-  double acc[4] = {0, 0, 0, 0};
-  for (int c0 = s0; c0 < s1; c0 += NA_TILE) {
-    const int cnt = min(NA_TILE, s1 - c0);
-    __syncthreads();
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      const size_t p = (size_t)(c0 + j);
-      sx[j] = spos[3 * p];
-      sy[j] = spos[3 * p + 1];
-      sz[j] = spos[3 * p + 2];
-      nx[j] = snor[3 * p];
-      ny[j] = snor[3 * p + 1];
-      nz[j] = snor[3 * p + 2];
-      for (int s = 0; s < SD; s++) f[j * SD + s] = sden[p * SD + s];
-    }
-    __syncthreads();
-    if (t < nt)
-      for (int j = 0; j < cnt; j++) {
-        double nrm[3] = {nx[j], ny[j], nz[j]};
-        keval<KT, double>(px - sx[j], py - sy[j], pz - sz[j], nrm, &f[j * SD], acc, kc);
-      }
-  }
-  if (t < nt)
-    for (int d = 0; d < TD; d++) partial[((size_t)blockIdx.y * nt + t) * TD + d] = acc[d];
-}
-
-__global__ void k_direct_reduce(const double* __restrict__ partial, int nchunk, int n, double* __restrict__ out) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int c = 0; c < nchunk; c++) s += partial[(size_t)c * n + e];
-    out[e] = s;
-  }
-}
-
-template <int KT>
-void launch_partial(dim3 grid, cudaStream_t st, const double* spos, const double* snor, const double* sden, int ns,
-                    int chunk, const double* tpos, int nt, double* partial, const KConst<double>& kc) {
-  k_direct_partial<KT><<<grid, NA_THREADS, 0, st>>>(spos, snor, sden, ns, chunk, tpos, nt, partial, kc);
-}
 
 }  // namespace
 }  // namespace kifmm
@@ -143,26 +80,8 @@ extern "C" kifmm_status kifmm_direct_noalloc(int kt, int ncoef, const double* co
   double kcd[3], cf[2] = {1.0, 0.25};
   for (int i = 0; i < ncoef && i < 2; i++) cf[i] = coefs[i];
   kernel_constants(kt, cf, kcd);
-  KConst<double> kc{kcd[0], kcd[1], kcd[2]};
-  // chunks of sources: enough CTAs to fill the GPU, within the scratch capacity
-  const int tblocks = (nt + NA_THREADS - 1) / NA_THREADS;
-  int nchunk = (int)std::min<size_t>((size_t)NA_MAXCHUNK, (size_t)KIFMM_NOALLOC_SCRATCH_DOUBLES / per_chunk);
-  nchunk = std::max(1, std::min(nchunk, std::max(1, 4 * num_sms / tblocks)));
-  nchunk = std::max(1, std::min(nchunk, std::max(1, ns / NA_TILE)));
-  const int chunk = ns > 0 ? (ns + nchunk - 1) / nchunk : 0;
-  dim3 grid(tblocks, nchunk);
-  switch (kt) {
-    case 111: launch_partial<111>(grid, st, d_srcpos, d_srcnor, d_srcden, ns, chunk, d_trgpos, nt, scratch, kc); break;
-    case 121: launch_partial<121>(grid, st, d_srcpos, d_srcnor, d_srcden, ns, chunk, d_trgpos, nt, scratch, kc); break;
-    case 311: launch_partial<311>(grid, st, d_srcpos, d_srcnor, d_srcden, ns, chunk, d_trgpos, nt, scratch, kc); break;
-    case 312: launch_partial<312>(grid, st, d_srcpos, d_srcnor, d_srcden, ns, chunk, d_trgpos, nt, scratch, kc); break;
-    case 321: launch_partial<321>(grid, st, d_srcpos, d_srcnor, d_srcden, ns, chunk, d_trgpos, nt, scratch, kc); break;
-    case 322: launch_partial<322>(grid, st, d_srcpos, d_srcnor, d_srcden, ns, chunk, d_trgpos, nt, scratch, kc); break;
-    case 511: launch_partial<511>(grid, st, d_srcpos, d_srcnor, d_srcden, ns, chunk, d_trgpos, nt, scratch, kc); break;
-    case 521: launch_partial<521>(grid, st, d_srcpos, d_srcnor, d_srcden, ns, chunk, d_trgpos, nt, scratch, kc); break;
-  }
-  const int n = (int)per_chunk;
-  k_direct_reduce<<<std::max(1, std::min((n + 255) / 256, num_sms * 8)), 256, 0, st>>>(scratch, nchunk, n, d_trgval);
+  const DirectPlan plan = direct_plan(ns, nt, td, num_sms, (size_t)KIFMM_NOALLOC_SCRATCH_DOUBLES);
+  launch_direct(kt, plan, d_srcpos, d_srcnor, d_srcden, ns, d_trgpos, nt, d_trgval, scratch, kcd, num_sms, st);
   if (cudaGetLastError() != cudaSuccess) return KIFMM_ERR_CUDA;
   return KIFMM_OK;
 }

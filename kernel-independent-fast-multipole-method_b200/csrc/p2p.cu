@@ -6,7 +6,6 @@
 //                       upward equivalent surfaces (UE2TC_dgemv, :114-141) and L2T from the leaf's own
 //                       downward equivalent surface (DE2TC_dgemv, :84-112), fused into one pass that
 //                       writes each target once.
-//   k_direct          : FP64 direct sum (Dense3d::eval, fmm3d/dense3d.cpp:38-57).
 //
 // S2M and the leaf pass run one warp per leaf (see below); S2L, rare, one CTA
 // per node with shared-memory tiles.  Every target accumulates in registers.
@@ -375,14 +374,17 @@ __global__ void __launch_bounds__(32 * WP_WARPS) k_s2m_warp(P2PArgs<T> a, const 
   }
 }
 
-// Leaf pass: the leaf's targets in rounds of up to 32; in a round lane =
-// (target slot, source split) with G = the power of two >= the round's
+// Leaf pass, one warp per work item: a round of up to 32 targets of one leaf
+// against a range of the leaf's sources (leaf_items below cuts long ranges).
+// lane = (target slot, source split) with G = the power of two >= the round's
 // target count (<= 32) slots and 32 / G splits, so a leaf of 33-64 targets
 // splits its last round's sources over the lanes its few targets leave;
-// splits are summed with warp shuffles.  Sources are staged 32 at a time: point
+// splits are summed with warp shuffles.  Sources are staged 64 at a time: point
 // sources from the leaf's near list (segments = source leaves, found by
 // bisection of the warp's prefix sums), then the W-list upward equivalent
-// surfaces and the leaf's own downward equivalent surface.
+// surfaces and the leaf's own downward equivalent surface.  An item of a cut
+// range writes partial[out][slot][d] (T, the accumulator's type), which
+// k_leaf_reduce adds up in item order.
 template <typename T>
 struct WarpSegs {
   int beg[32];
@@ -393,9 +395,9 @@ struct WarpSegs {
 };
 
 template <typename T, int KT, int NWARP>
-__global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const int* work, const int64_t* nptr,
-                                                             const int* nidx, const int64_t* mptr, const int* midx,
-                                                             int nwork, int rhs) {
+__global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const LeafItem* __restrict__ items,
+                                                          const int* __restrict__ nidx, const int* __restrict__ midx,
+                                                          int nitem, T* __restrict__ partial, int rhs) {
   constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD;
   constexpr bool DL = KTraits<KT>::DL;
   constexpr int MM = KTraits<KT>::MM;
@@ -408,22 +410,22 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const in
   // packed FP32 Laplace sums (near field for KT 111, surfaces for MM 111)
   constexpr bool PAIR_NEAR = KT == 111 && sizeof(T) == 4, PAIR_SURF = MM == 111 && sizeof(T) == 4;
   const T* den = a.sden + (size_t)rhs * a.ns * SD;
-  T* outbase = a.tval + (size_t)rhs * a.nt * TD;
   const int nsurf = a.nsurf;
-  for (int wi = blockIdx.x * NWARP + warp; wi < nwork; wi += gridDim.x * NWARP) {
-    const int g = work[wi];
+  for (int wi = blockIdx.x * NWARP + warp; wi < nitem; wi += gridDim.x * NWARP) {
+    const LeafItem it = items[wi];
+    const int g = it.g;
     const double cx = a.center[3 * g], cy = a.center[3 * g + 1], cz = a.center[3 * g + 2];
     const T rad = (T)a.radius[g];
     const int tb0 = a.tbeg[g], nt = a.tcnt[g];
-    const bool l2t = a.depth[g] >= a.l2t_depth;
-    const int64_t nb = nptr[wi], ne = nptr[wi + 1];
-    const int64_t mb = mptr[wi], me = mptr[wi + 1];
-    const int nsurf_segs = (int)(me - mb) + (l2t ? 1 : 0);
-    for (int tb = 0, G = 32; tb < nt; tb += G) {
-      G = 1;
-      while (G < nt - tb && G < 32) G <<= 1;
+    const int64_t nb = it.nb, ne = it.nb + it.nn;
+    const int64_t mb = it.mb, me = it.mb + it.nm;
+    const int nsurf_segs = it.nm + it.l2t;
+    int left = it.take;  // point sources of this item still to come
+    {
+      int G = 1;
+      while (G < nt - it.tb && G < 32) G <<= 1;
       const int nsplit = 32 / G, slot = lane % G, sg = lane / G;
-      const int ti = tb + slot;
+      const int ti = it.tb + slot;
       const bool valid = ti < nt;
       T px = 0, py = 0, pz = 0;
       if (valid) {
@@ -439,8 +441,9 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const in
         int cntl = 0;
         if (lane < nseg) {
           const int s = nidx[c0 + lane];
-          sgt.beg[lane] = a.sbeg[s];
-          cntl = a.scnt[s];
+          const int skip = c0 == nb && lane == 0 ? it.skip : 0;  // the item begins inside its first leaf
+          sgt.beg[lane] = a.sbeg[s] + skip;
+          cntl = a.scnt[s] - skip;
           sgt.shx[lane] = (T)(a.center[3 * s] - cx);
           sgt.shy[lane] = (T)(a.center[3 * s + 1] - cy);
           sgt.shz[lane] = (T)(a.center[3 * s + 2] - cz);
@@ -454,7 +457,8 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const in
         }
         sgt.pre[lane + 1] = incl;
         if (lane == 0) sgt.pre[0] = 0;
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        const int total = min(left, __shfl_sync(0xffffffffu, incl, 31));
+        left -= total;
         __syncwarp();
         for (int k0 = 0; k0 < total; k0 += 64) {
           const int cnt = min(64, total - k0);
@@ -501,7 +505,7 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const in
                 const P4<T> s = w.p[sg + r * nsplit];
                 const T x = px - s.x, y = py - s.y, z = pz - s.z;
                 const T r2 = x * x + y * y + z * z;
-                const T ri = (r2 >= T(1e-16)) ? rsqrt_t(r2) : T(0);
+                const T ri = rinv_cut(r2);
                 s1 += ri * s.w;
               }
               acc[0] += a.ku.c0 * s1;
@@ -584,7 +588,7 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const in
                 const P4<T> s = w.p[sg + r * nsplit];
                 const T x = px - s.x, y = py - s.y, z = pz - s.z;
                 const T r2 = x * x + y * y + z * z;
-                const T ri = (r2 >= T(1e-16)) ? rsqrt_t(r2) : T(0);
+                const T ri = rinv_cut(r2);
                 s1 += ri * s.w;
               }
               acc[0] += a.km.c0 * s1;
@@ -609,50 +613,28 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const in
 #pragma unroll
       for (int d = 0; d < TD; d++)
         for (int o = G; o < 32; o <<= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
-      if (valid && sg == 0)
+      if (valid && sg == 0) {
+        T* o = it.out >= 0 ? partial + ((size_t)it.out * 32 + slot) * TD
+                           : a.tval + ((size_t)rhs * a.nt + tb0 + ti) * TD;
 #pragma unroll
-        for (int d = 0; d < TD; d++) outbase[(size_t)(tb0 + ti) * TD + d] = acc[d];
+        for (int d = 0; d < TD; d++) o[d] = acc[d];
+      }
     }
   }
 }
 
-// FP64 direct sum over all sources, absolute coordinates (3 x n interleaved).
-template <int KT>
-__global__ void __launch_bounds__(P2P_THREADS) k_direct(const double* spos, const double* snor, const double* sden,
-                                                         int ns, const double* tpos, int nt, double* out,
-                                                         KConst<double> kc) {
-  constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD;
-  __shared__ double sx[TILE], sy[TILE], sz[TILE], nx[TILE], ny[TILE], nz[TILE], f[TILE * 4];
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  double px = 0, py = 0, pz = 0;
-  if (t < nt) {
-    px = tpos[3 * t];
-    py = tpos[3 * t + 1];
-    pz = tpos[3 * t + 2];
-  }
-  double acc[4] = {0, 0, 0, 0};
-  for (int c0 = 0; c0 < ns; c0 += TILE) {
-    int cnt = min(TILE, ns - c0);
-    __syncthreads();
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      int p = c0 + j;
-      sx[j] = spos[3 * p];
-      sy[j] = spos[3 * p + 1];
-      sz[j] = spos[3 * p + 2];
-      nx[j] = snor[3 * p];
-      ny[j] = snor[3 * p + 1];
-      nz[j] = snor[3 * p + 2];
-      for (int s = 0; s < SD; s++) f[j * SD + s] = sden[(size_t)p * SD + s];
-    }
-    __syncthreads();
-    if (t < nt)
-      for (int j = 0; j < cnt; j++) {
-        double nrm[3] = {nx[j], ny[j], nz[j]};
-        keval<KT, double>(px - sx[j], py - sy[j], pz - sz[j], nrm, &f[j * SD], acc, kc);
-      }
-  }
-  if (t < nt)
-    for (int d = 0; d < TD; d++) out[(size_t)t * TD + d] = acc[d];
+// tval of one round = the sum of its items' partial potentials, in item order
+template <typename T, int TD>
+__global__ void k_leaf_reduce(const LeafSplit* __restrict__ splits, int n, const T* __restrict__ partial,
+                              T* __restrict__ tval) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, w = e / (32 * TD), k = e % (32 * TD);
+  if (w >= n) return;
+  const LeafSplit sp = splits[w];
+  if (k >= sp.cnt * TD) return;
+  T s = T(0);
+#pragma unroll 4
+  for (int p = 0; p < sp.parts; p++) s += partial[((size_t)(sp.first + p) * 32) * TD + k];
+  tval[(size_t)sp.tbeg * TD + k] = s;
 }
 
 // sden_sorted[r][i][s] = srcden[r][perm[i]][s]
@@ -712,14 +694,112 @@ void launch_p2p_kt(const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cu
     case P2P_LEAF:
       if (w.n) {
         constexpr int nw = sizeof(T) == 4 ? 8 : 4;  // static shared memory: 64 staged sources per warp
-        const int grid = std::min((w.n + nw - 1) / nw, 148 * 32);
-        k_leaf_warp<T, KT, nw><<<grid, 32 * nw, 0, st>>>(a, w.work, w.ptr, w.idx, w.ptr2, w.idx2, w.n, rhs);
+        const int grid = std::min((w.nitem + nw - 1) / nw, 148 * 32);
+        k_leaf_warp<T, KT, nw>
+            <<<grid, 32 * nw, 0, st>>>(a, w.items, w.idx, w.idx2, w.nitem, static_cast<T*>(w.partial), rhs);
+        if (w.nsplit > 0) {
+          constexpr int TD = KTraits<KT>::TD;
+          k_leaf_reduce<T, TD><<<(w.nsplit * 32 * TD + 255) / 256, 256, 0, st>>>(
+              w.splits, w.nsplit, static_cast<const T*>(w.partial), a.tval + (size_t)rhs * a.nt * TD);
+        }
       }
       break;
   }
 }
 
 }  // namespace
+
+// Work items of the leaf pass.  One warp per leaf, the form before, left a
+// leaf with long lists to one warp (150,001 sources on an ellipsoid, targets
+// in the volume: the coarse leaves' W lists hold hundreds of surfaces, 17.9 ms
+// in that warp's tail) and a small tree's leaves on a few SMs (2,000 points:
+// 56 warps, 0.15 ms).  A range costs its sources over the lanes that share a
+// target; it is cut above `limit` = 1/8 of a warp's share when every SM holds
+// 32 warps, and not below `least` sources (two staged batches in FP64, four in
+// FP32, whose pairs take a quarter of the time), where starting an item and
+// adding its partial sum would cost more than the sources.
+void leaf_items(int nwork, const int* work, const int* tcnt, const int* scnt, const int64_t* nptr, const int* nidx,
+                const int64_t* mptr, const unsigned char* l2t, const int* tbeg, int nsurf, int least, int num_sms,
+                std::vector<LeafItem>* items, std::vector<LeafSplit>* splits, int* nparts) {
+  items->clear();
+  splits->clear();
+  *nparts = 0;
+  auto lanes = [](int left) {  // lanes that share a target in a round with `left` targets to go
+    int G = 1;
+    while (G < left && G < 32) G <<= 1;
+    return 32 / G;
+  };
+  std::vector<int64_t> nsrc(nwork);
+  double total = 0;
+  for (int w = 0; w < nwork; w++) {
+    int64_t s = 0;
+    for (int64_t k = nptr[w]; k < nptr[w + 1]; k++) s += scnt[nidx[k]];
+    nsrc[w] = s;
+    const int nt = tcnt[work[w]];
+    const double all = (double)s + (double)nsurf * ((mptr[w + 1] - mptr[w]) + l2t[w]);
+    for (int tb = 0; tb < nt; tb += 32) total += all / lanes(nt - tb);
+  }
+  const double limit = std::max((double)least, total / ((double)num_sms * 32 * 8));
+  for (int w = 0; w < nwork; w++) {
+    const int g = work[w], nt = tcnt[g];
+    const int nseg = (int)(mptr[w + 1] - mptr[w]) + l2t[w];
+    const int64_t all = nsrc[w] + (int64_t)nseg * nsurf;
+    for (int tb = 0; tb < nt; tb += 32) {
+      const double cost = (double)all / lanes(nt - tb);
+      const int parts = cost > 1.5 * limit ? (int)std::min(cost / limit + 0.5, 65536.0) : 1;
+      int64_t seg = nptr[w];  // the near segment the next item begins in, `skip` sources into it
+      int skip = 0, s0 = 0;   // and its first surface
+      int64_t k0 = 0;
+      const int first = *nparts;
+      int made = 0;
+      for (int p = 0; p < parts; p++) {
+        const bool last = p + 1 == parts;
+        const int64_t cut = last ? all : (int64_t)((double)all * (p + 1) / parts);
+        const int64_t k1 = last ? nsrc[w] : std::max(k0, std::min(nsrc[w], (cut + 63) / 64 * 64));
+        int s1 = last ? nseg : std::max(s0, (int)((std::max(cut, nsrc[w]) - nsrc[w]) / nsurf));
+        if (k1 == k0 && s1 == s0 && !(last && made == 0)) continue;
+        LeafItem it;
+        it.g = g;
+        it.tb = tb;
+        it.nb = seg;
+        it.skip = skip;
+        it.take = (int)(k1 - k0);
+        int64_t left = k1 - k0;
+        int64_t e = seg;
+        while (left > 0) {
+          const int64_t c = scnt[nidx[e]] - skip;
+          if (left < c) {
+            skip += (int)left;
+            left = 0;
+            break;
+          }
+          left -= c;
+          skip = 0;
+          e++;
+        }
+        it.nn = (int)(e - seg) + (skip > 0 ? 1 : 0);
+        if (it.take == 0) it.nn = 0;
+        seg = e;
+        it.mb = mptr[w] + s0;
+        it.l2t = s1 == nseg && s1 > s0 ? l2t[w] : 0;
+        it.nm = s1 - s0 - it.l2t;
+        it.out = parts > 1 ? (*nparts)++ : -1;
+        made++;
+        k0 = k1;
+        s0 = s1;
+        items->push_back(it);
+      }
+      if (parts > 1) {
+        if (made == 1) {  // nothing was cut after all
+          items->back().out = -1;
+          (*nparts)--;
+        } else {
+          splits->push_back(LeafSplit{tbeg[g] + tb, std::min(32, nt - tb), first, made});
+        }
+      }
+    }
+  }
+}
 
 template <typename T>
 void launch_p2p(int kt, const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cudaStream_t st) {
@@ -736,23 +816,6 @@ void launch_p2p(int kt, const P2PArgs<T>& a, const P2PWork& w, int which, int rh
 }
 template void launch_p2p<double>(int, const P2PArgs<double>&, const P2PWork&, int, int, cudaStream_t);
 template void launch_p2p<float>(int, const P2PArgs<float>&, const P2PWork&, int, int, cudaStream_t);
-
-void launch_direct(int kt, const double* spos, const double* snor, const double* sden, int ns, const double* tpos,
-                   int nt, double* out, const double* kc3, cudaStream_t st) {
-  KConst<double> kc{kc3[0], kc3[1], kc3[2]};
-  int grid = (nt + P2P_THREADS - 1) / P2P_THREADS;
-  if (grid == 0) return;
-  switch (kt) {
-    case 111: k_direct<111><<<grid, P2P_THREADS, 0, st>>>(spos, snor, sden, ns, tpos, nt, out, kc); break;
-    case 121: k_direct<121><<<grid, P2P_THREADS, 0, st>>>(spos, snor, sden, ns, tpos, nt, out, kc); break;
-    case 311: k_direct<311><<<grid, P2P_THREADS, 0, st>>>(spos, snor, sden, ns, tpos, nt, out, kc); break;
-    case 312: k_direct<312><<<grid, P2P_THREADS, 0, st>>>(spos, snor, sden, ns, tpos, nt, out, kc); break;
-    case 321: k_direct<321><<<grid, P2P_THREADS, 0, st>>>(spos, snor, sden, ns, tpos, nt, out, kc); break;
-    case 322: k_direct<322><<<grid, P2P_THREADS, 0, st>>>(spos, snor, sden, ns, tpos, nt, out, kc); break;
-    case 511: k_direct<511><<<grid, P2P_THREADS, 0, st>>>(spos, snor, sden, ns, tpos, nt, out, kc); break;
-    case 521: k_direct<521><<<grid, P2P_THREADS, 0, st>>>(spos, snor, sden, ns, tpos, nt, out, kc); break;
-  }
-}
 
 template <typename T>
 void launch_scatter_den(const double* srcden, const int* perm, int ns, int sd, int nrhs, T* out, cudaStream_t st) {
