@@ -89,6 +89,45 @@ std::shared_ptr<Tc16Images> tc16_images(const std::shared_ptr<const Operators>& 
   return p;
 }
 
+// The operator tables of the FP64 Hadamard, shared and freed in the same way (Navier np = 8: 207 MB).
+struct Had64Tables {
+  double* t = nullptr;
+  int device = 0;
+  ~Had64Tables() {
+    int cur = 0;
+    cudaGetDevice(&cur);
+    if (cur != device) cudaSetDevice(device);
+    if (t) cudaFree(t);
+    if (cur != device) cudaSetDevice(cur);
+  }
+};
+
+std::shared_ptr<Had64Tables> had64_tables(const std::shared_ptr<const Operators>& ops, int device, int nf, int sd,
+                                          int td, int num_sms) {
+  static std::mutex mu;
+  static std::map<std::pair<const Operators*, int>, std::pair<std::weak_ptr<const Operators>, std::weak_ptr<Had64Tables>>>
+      cache;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_pair(ops.get(), device);
+  auto it = cache.find(key);
+  if (it != cache.end() && !it->second.first.expired())
+    if (auto p = it->second.second.lock()) return p;
+  auto p = std::make_shared<Had64Tables>();
+  p->device = device;
+  KCHECK(cudaMalloc(&p->t, had64_table_doubles(nf, sd, td) * sizeof(double)));
+  double* khat = nullptr;
+  KCHECK(cudaMalloc(&khat, ops->m2l.size() * 2 * sizeof(double)));
+  cudaError_t e = cudaMemcpy(khat, ops->m2l.data(), ops->m2l.size() * 2 * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    launch_had64_tables(khat, nf, sd, td, p->t, num_sms, 0);
+    e = cudaStreamSynchronize(0);  // other engines' streams do not wait for the default stream
+  }
+  cudaFree(khat);
+  if (e != cudaSuccess) throw CudaError{e, "FP64 Hadamard tables"};
+  cache[key] = std::make_pair(std::weak_ptr<const Operators>(ops), std::weak_ptr<Had64Tables>(p));
+  return p;
+}
+
 }  // namespace
 
 template <typename T>
@@ -183,7 +222,7 @@ struct Impl : ImplBase {
   T *ybuf, *zbuf;  // per-node rank-space coordinates of the upward / downward densities
   int ru = 0, rd = 0;  // ranks rounded up to multiples of 8 (zero-padded rows / columns)
   bool use_tc = false;
-  T* khat;
+  T* khat = nullptr;     // [343][td][sd][nf], np other than 4, 6, 8
   T* ktiles = nullptr;  // [td][sd][ceil(nf/32)][343][32] operator spectra for the parent-pair sweep
   T* ttiles = nullptr;  // [td][sd][ceil(nf/16)][26][27][16] Toeplitz-factored operator
   float* htc_img = nullptr;         // tensor-core Hadamard (split TF32): operator images per (4 frequencies, direction)
@@ -193,6 +232,9 @@ struct Impl : ImplBase {
   unsigned* d_bound = nullptr;          // ... and the per-eval bound of the spectra (FP32 bits)
   int* htc16_ctab = nullptr;            // ... and its colleague tables [tile][26][128]
   bool htc() const { return htc_img || htc16_img; }
+  const double* had64 = nullptr;        // FP64 Toeplitz-factored Hadamard: transformed operator
+  std::shared_ptr<Had64Tables> had64_shared;  // ... held from the per-device cache
+  Had64Groups had64_grp;                // ... and its groups of target parents
   unsigned* htc_dirs = nullptr;     // tensor-core Hadamard: directions present per tile of 128 parents
   int* h_status = nullptr;  // mapped host word: device-side wait time-outs (bit 0 sweep, bit 1 GEMM, bit 2 TC Hadamard)
   int* d_status = nullptr;
@@ -300,43 +342,36 @@ struct Impl : ImplBase {
     args.de_unit = upload_as_T(op.de);
     args.dc_unit = upload_as_T(op.dc);
     build_surface_ops();
-    {
+    KCHECK(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, E.device));
+    if (m2l_sweep_supported(op.nfc, sd_m, td_m)) {
+      if (sizeof(T) == 4 && E.m2l_tc && !E.m2l_tc_tf32 && m2l_tc16_supported(op.nfc, sd_m, td_m)) {
+        htc16_shared = tc16_images(E.ops, E.device, op.nfc, sd_m, td_m);
+        htc16_img = htc16_shared->img;
+        htc16_inv_sb = htc16_shared->inv_sb;
+      } else if (sizeof(T) == 4 && E.m2l_tc && m2l_tc_supported(op.nfc, sd_m, td_m)) {
+        std::vector<float> im;
+        m2l_tc_images(op.nfc, op.m2l.data(), &im);
+        htc_img = upload(im);
+      } else if (E.m2l_toeplitz) {
+        if (sizeof(T) == 8) {
+          had64_shared = had64_tables(E.ops, E.device, op.nfc, sd_m, td_m, num_sms);
+          had64 = had64_shared->t;
+        } else {
+          ttiles = upload(toeplitz_tables());
+        }
+      } else if (E.per_level) {  // one set of operator tiles per level
+        for (auto& lo : E.lops->ops) ktiles_lv.push_back(upload(sweep_tiles(*lo)));
+        ktiles = ktiles_lv[0];
+      } else {
+        ktiles = upload(sweep_tiles(op));
+      }
+    } else {  // np other than 4, 6, 8: one V list per node
       std::vector<T> kh(op.m2l.size() * 2);
       for (size_t i = 0; i < op.m2l.size(); i++) {
         kh[2 * i] = (T)op.m2l[i].real();
         kh[2 * i + 1] = (T)op.m2l[i].imag();
       }
       khat = upload(kh);
-      if (m2l_sweep_supported(op.nfc, sd_m, td_m)) {
-        // [td][sd][ftile][343][32]; the spectra are [343][td][sd][nf]
-        const int nf = op.nfc, ftiles = (nf + 31) / 32, tsd = td_m * sd_m;
-        std::vector<T> kt((size_t)tsd * ftiles * 343 * 32 * 2, T(0));
-        for (int ts = 0; ts < tsd; ts++)
-          for (int ft = 0; ft < ftiles; ft++)
-            for (int o = 0; o < 343; o++)
-              for (int l = 0; l < 32 && ft * 32 + l < nf; l++) {
-                const size_t dst = ((((size_t)ts * ftiles + ft) * 343 + o) * 32 + l) * 2;
-                const size_t src = (((size_t)o * tsd + ts) * nf + ft * 32 + l) * 2;
-                kt[dst] = kh[src];
-                kt[dst + 1] = kh[src + 1];
-              }
-        if (sizeof(T) == 4 && E.m2l_tc && !E.m2l_tc_tf32 && m2l_tc16_supported(nf, sd_m, td_m)) {
-          htc16_shared = tc16_images(E.ops, E.device, nf, sd_m, td_m);
-          htc16_img = htc16_shared->img;
-          htc16_inv_sb = htc16_shared->inv_sb;
-        } else if (sizeof(T) == 4 && E.m2l_tc && m2l_tc_supported(nf, sd_m, td_m)) {
-          std::vector<float> im;
-          m2l_tc_images(nf, op.m2l.data(), &im);
-          htc_img = upload(im);
-        } else if (E.m2l_toeplitz) {
-          ttiles = upload(toeplitz_tables());
-        } else if (E.per_level) {  // one set of operator tiles per level
-          for (auto& lo : E.lops->ops) ktiles_lv.push_back(upload(sweep_tiles(*lo)));
-          ktiles = ktiles_lv[0];
-        } else {
-          ktiles = upload(kt);
-        }
-      }
     }
     KCHECK(cudaHostAlloc((void**)&h_status, sizeof(int), cudaHostAllocMapped));
     *h_status = 0;
@@ -418,7 +453,6 @@ struct Impl : ImplBase {
         off_up = level_offsets(all_up_lvl, md);
         off_dn = level_offsets(all_dn_lvl, md);
       }
-      KCHECK(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, E.device));
       gemm_ws_len = (size_t)4 << 20;  // split-K slices of the shallow levels (32 MB)
       gemm_ws = dalloc<double>(gemm_ws_len);
     }
@@ -449,11 +483,12 @@ struct Impl : ImplBase {
       // 8 blocks from index nn on stand for an absent colleague (parent-pair form)
       // (tensor-core form: sibling-group major, node n in group (n + 7) / 8,
       // the zero block a group of its own: (nn + 15) / 8 groups of 8 nodes)
-      // (FP16 form, several source dofs: one such plane per dof)
-      S_spec = std::max((size_t)(nn + 8) * sd_m, htc() ? (size_t)(nn + 15) / 8 * 8 * (htc16_img ? sd_m : 1) : 0) *
+      // (FP16 and FP64 forms, several source dofs: one such plane per dof)
+      S_spec = std::max((size_t)(nn + 8) * sd_m,
+                        htc() || had64 ? (size_t)(nn + 15) / 8 * 8 * (htc_img ? 1 : sd_m) : 0) *
                op.nfc * 2;
       counters_v = (double)idx.size();
-      if (ktiles || ttiles || htc()) build_pairs(work);
+      if (!khat) build_pairs(work);
       counters_fwd = (double)fwdn.size();
       counters_inv = (double)work.size();
     }
@@ -526,9 +561,9 @@ struct Impl : ImplBase {
     geom.td = td_m;
     for (int s = 0; s < sd_m && s < 4; s++) geom.deg[s] = E.per_level ? 0 : op.deg[s];
     geom.rootlvl = E.rootlvl;
-    geom.sg = htc16_img ? 2 : htc_img ? 1 : 0;
-    geom.effval_sg = htc16_img ? 1 : 0;
-    geom.plane = htc16_img ? (size_t)((nn + 15) / 8 * 8) * op.nfc : 0;
+    geom.sg = htc16_img ? 2 : htc_img || had64 ? 1 : 0;
+    geom.effval_sg = htc16_img || had64 ? 1 : 0;
+    geom.plane = htc16_img || had64 ? (size_t)((nn + 15) / 8 * 8) * op.nfc : 0;
     geom.bound = d_bound;
     scl.sd = sd_m;
     for (int s = 0; s < sd_m && s < 4; s++) scl.deg[s] = E.per_level ? 0 : op.deg[s];
@@ -722,7 +757,6 @@ struct Impl : ImplBase {
 
   void build_pairs(const std::vector<int>& vtargets) {
     const Csr& V = tr.lists[1];
-    KCHECK(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, E.device));
     // one work item per target parent of a node with a V list
     std::vector<int> qlist;
     std::vector<char> seen(tr.nnodes, 0);
@@ -758,10 +792,16 @@ struct Impl : ImplBase {
         }
       }
     }
+    pairs_n = (int)qlist.size();
+    if (had64) {
+      Had64HostGroups h;
+      had64_groups(pairs_n, tr.nnodes, qchd.data(), coll.data(), &h);
+      had64_grp = Had64Groups{upload(h.head), upload(h.tab), upload(h.desc), upload(h.out)};
+      return;
+    }
     pairs_chd = upload(qchd);
     pairs_coll = upload(coll);
     pairs_mask = upload(mask);
-    pairs_n = (int)qlist.size();
     if (htc()) {  // directions present per tile of 128 target parents (an empty tile keeps one)
       std::vector<unsigned> dirs((pairs_n + 127) / 128, 0u);
       double steps = 0;
@@ -964,6 +1004,10 @@ struct Impl : ImplBase {
       launch_m2l_hadamard_tc(op.nfc, htc_img, reinterpret_cast<const float*>(spec), pairs_n, pairs_chd, pairs_coll,
                              pairs_mask, htc_dirs, reinterpret_cast<float*>(eff), tr.nnodes, d_status, num_sms, st);
       KCHECK(cudaGetLastError());
+    } else if (pairs_n > 0 && had64) {
+      if constexpr (sizeof(T) == 8)
+        launch_m2l_hadamard64(op.nfc, sd_m, td_m, had64, spec, geom.plane, pairs_n, had64_grp, eff, num_sms,
+                              st);
     } else if (pairs_n > 0 && E.per_level) {
       // parents by depth d, their children's V lists with level d + 1's operators
       for (int d = 0; d + 1 < (int)ktiles_lv.size(); d++) {
@@ -973,19 +1017,19 @@ struct Impl : ImplBase {
                                        pairs_coll + (size_t)b * 26, pairs_mask + b, eff, tr.nnodes, d_status, num_sms,
                                        st);
       }
+    } else if (pairs_n > 0 && ttiles) {
+      if constexpr (sizeof(T) == 4)
+        launch_m2l_hadamard_tz(op.nfc, sd_m, td_m, ttiles, spec, pairs_n, pairs_chd, pairs_coll, pairs_mask, eff,
+                               tr.nnodes, d_status, num_sms, st);
     } else if (pairs_n > 0) {
-      if (ttiles)
-        launch_m2l_hadamard_tz<T>(op.nfc, sd_m, td_m, ttiles, spec, pairs_n, pairs_chd, pairs_coll, pairs_mask, eff,
-                                  tr.nnodes, d_status, num_sms, st);
-      else
-        launch_m2l_hadamard_sweep<T>(op.nfc, sd_m, td_m, ktiles, spec, pairs_n, pairs_chd, pairs_coll, pairs_mask,
-                                     eff, tr.nnodes, d_status, num_sms, st);
+      launch_m2l_hadamard_sweep<T>(op.nfc, sd_m, td_m, ktiles, spec, pairs_n, pairs_chd, pairs_coll, pairs_mask, eff,
+                                   tr.nnodes, d_status, num_sms, st);
     } else {
       launch_m2l_hadamard<T>(g, khat, spec, m2l.work, m2l.n, m2l.ptr, m2l.idx, d_path, eff, st);
     }
     if (prof) KCHECK(cudaEventRecord(ev[8], st));
     launch_m2l_inverse<T>(g, eff, m2l.work, m2l.n, tdc, st);
-    nlaunch += 2 + (pairs_n > 0 ? (htc() ? 1 : sd_m * td_m) : 1);
+    nlaunch += 2 + (pairs_n > 0 && !htc() && !had64 ? sd_m * td_m : 1);
   }
 
   // Density vectors go through the passes in chunks of up to max_chunk: the
@@ -1210,10 +1254,9 @@ int Engine::setup() {
     }
     tensor_cores = tc != 0;
     auto fit = opts.find("-" + prefix + "m2l_form");
-    // default: in mixed precision the tensor-core form for single-dof kernels
-    // (tensor_cores on), else the factored form (as fast as the direct form
-    // with ~40 % fewer multiply-adds); the direct form in FP64 (faster there)
-    m2l_toeplitz = mixed;
+    // default: in mixed precision the tensor-core form (tensor_cores on), else
+    // and in FP64 the factored form (~40 % fewer multiply-adds than the direct)
+    m2l_toeplitz = true;
     m2l_tc = mixed && tensor_cores;
     m2l_tc_tf32 = false;
     int wl = 1 << 22;

@@ -152,10 +152,11 @@ struct M2LGeom {
   int deg[4] = {0, 0, 0, 0};
   int rootlvl = 0;
   // 2: the sibling-group-major layout holding FP16 pairs (below)
-  // 0: spectra[node][s][f]; 1 (single dof): sibling-group major,
-  // spectra[(node + 7) / 8][f / 4][(node + 7) % 8][f % 4] -- every sibling
+  // 0: spectra[node][s][f]; 1: sibling-group major, one plane per dof,
+  // spectra[s][(node + 7) / 8][f / 4][(node + 7) % 8][f % 4] -- every sibling
   // group's spectra one block, and in it the 8 children's values of 4
-  // frequencies 256 contiguous bytes (first children are 1 mod 8)
+  // frequencies contiguous (first children are 1 mod 8); in FP64 those of 2
+  // (spectra_f64_index)
   int sg = 0;
   // sg == 2: each complex value x is stored as the FP16 pairs
   // {hi(re), hi(im)}, {lo(re), lo(im)} of x * 2^(14 - e), where 2^e >= the
@@ -164,17 +165,21 @@ struct M2LGeom {
   // would take
   const unsigned* bound = nullptr;
   // accumulated spectra in the sibling-group-major layout of
-  // spectra_sg_index instead of [node][td][nfc] (written so by the FP16
-  // tensor-core Hadamard)
+  // sg 1 or 2 instead of [node][td][nfc] (written so by the FP16
+  // tensor-core and the FP64 Hadamard)
   int effval_sg = 0;
-  // sg == 2 and effval_sg: complex slots per dof plane of the
-  // sibling-group-major spectra (dof s at s * plane + spectra_sg_index)
+  // complex slots per dof plane of the sibling-group-major spectra (dof s at
+  // s * plane + spectra_sg_index)
   size_t plane = 0;
 };
 // complex index of (node, compact frequency c) in the sibling-group-major
 // layout of nfc frequencies (a multiple of 4)
 __host__ __device__ inline size_t spectra_sg_index(int nfc, int node, int c) {
   return (((size_t)((node + 7) >> 3) * (nfc >> 2) + (c >> 2)) * 8 + ((node + 7) & 7)) * 4 + (c & 3);
+}
+// complex index in the FP64 form's layout: [sibling group][f / 2][8 children][f % 2]
+__host__ __device__ inline size_t spectra_f64_index(int nfc, int node, int c) {
+  return (((size_t)((node + 7) >> 3) * (nfc >> 1) + (c >> 1)) * 8 + ((node + 7) & 7)) * 2 + (c & 1);
 }
 
 // spectra[node][s][f] (complex, interleaved re/im) of 2^(l*deg) * supeden[node]
@@ -198,14 +203,32 @@ void launch_m2l_hadamard_sweep(int nf, int sd, int td, const T* ktiles, const T*
                                const int* coll, const unsigned char* mask, T* effval, int zero_node, int* status,
                                int num_sms, cudaStream_t st);
 // The same product with the 2 x 2 x 2 block-Toeplitz factorisation of each
-// colleague block (27 instead of 64 complex products per direction).  ttiles:
-// [td][sd][ceil(nf/16)][26 directions][14][16][2] complex: for direction d
+// colleague block (27 instead of 64 complex products per direction), FP32.
+// ttiles: [td][sd][ceil(nf/16)][26 directions][14][16][2] complex: for direction d
 // and frequency lane l, the 27 transformed values k (padded to 28) stored as
 // pairs (k, k+1) at [d][k/2][l][k%2].
-template <typename T>
-void launch_m2l_hadamard_tz(int nf, int sd, int td, const T* ttiles, const T* spectra, int nq, const int* qchd,
-                            const int* coll, const unsigned char* mask, T* effval, int zero_node, int* status,
+void launch_m2l_hadamard_tz(int nf, int sd, int td, const float* ttiles, const float* spectra, int nq, const int* qchd,
+                            const int* coll, const unsigned char* mask, float* effval, int zero_node, int* status,
                             int num_sms, cudaStream_t st);
+// The FP64 form (m2l_f64.cu): spectra and accumulated spectra in the
+// layout of spectra_f64_index, one plane per dof.  Tables [td][nf][sd][26][27] complex, had64_table_doubles doubles, made on
+// the device from the operator spectra khat [343][td][sd][nf].  Parents in groups
+// of 16 rows, a step per direction that one of them has: head [group] {first
+// step, number of steps}, tab [step][16] the colleague's sibling group (the
+// all-zero group for an absent one or a padding row), desc [step] the operator
+// fragment and which 8 rows have the direction, out [group][16] the target
+// sibling group (-1: padding).
+struct Had64Groups {
+  const int *head = nullptr, *tab = nullptr, *desc = nullptr, *out = nullptr;
+};
+struct Had64HostGroups {
+  std::vector<int> head, tab, desc, out;
+};
+void had64_groups(int nq, int zero_node, const int* qchd, const int* coll, Had64HostGroups* o);
+size_t had64_table_doubles(int nf, int sd, int td);
+void launch_had64_tables(const double* khat, int nf, int sd, int td, double* tables, int num_sms, cudaStream_t st);
+void launch_m2l_hadamard64(int nf, int sd, int td, const double* tables, const double* spectra, size_t plane, int nq,
+                           const Had64Groups& g, double* effval, int num_sms, cudaStream_t st);
 // The same product for single-dof kernels in FP32 on the tensor cores
 // (m2l_tc.cu): tiles of 128 target parents, per frequency a split-TF32 MMA
 // with the gathered colleague spectra in TMEM; spectra in the

@@ -156,10 +156,7 @@ __global__ void __launch_bounds__(256) k_m2l_fwd_warp(M2LGeom g, const T* __rest
           r.re = fmt(-b.im, t.im, fmt(b.re, t.re, r.re));
           r.im = fmt(b.im, t.re, fmt(b.re, t.im, r.im));
         }
-        if (g.sg)
-          reinterpret_cast<Cpx<T>*>(spectra)[spectra_sg_index(nfc, node, c)] = r;
-        else
-          out[c] = r;
+        out[c] = r;  // (the sibling-group-major layouts need np = 4, 6 or 8)
       }
       __syncwarp();
     }
@@ -492,7 +489,9 @@ __global__ void __launch_bounds__(256) k_m2l_fwd_rb(M2LGeom g, const T* __restri
             }
           }
           if (g.sg)
-            reinterpret_cast<Cpx<T>*>(spectra)[spectra_sg_index(NFC, node, c)] = Cpx<T>{re, im};
+            reinterpret_cast<Cpx<T>*>(spectra)[s * g.plane + (sizeof(T) == 8 ? spectra_f64_index(NFC, node, c)
+                                                                              : spectra_sg_index(NFC, node, c))] =
+                Cpx<T>{re, im};
           else
             out[c] = Cpx<T>{re, im};
         }
@@ -537,7 +536,8 @@ __global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* __restri
       // warp's stage all at once, so the warp waits for memory once per node
       // (the stage was last read by the previous z pass, which ends in a
       // __syncwarp)
-      const Cpx<T>* srcg = reinterpret_cast<const Cpx<T>*>(effval) + t * g.plane + spectra_sg_index(NFC, node, 0);
+      const Cpx<T>* srcg = reinterpret_cast<const Cpx<T>*>(effval) + t * g.plane +
+                           (sizeof(T) == 8 ? spectra_f64_index(NFC, node, 0) : spectra_sg_index(NFC, node, 0));
       if constexpr (kStage) {
         if (stage_sg) {
           for (int b = lane; b < NFC / 4; b += 32) {
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* __restri
         for (int kz = 0; kz < N; kz++) {
           const int c = c_of[(kz * N + ky) * NH + kx];
           const int ca = c >= 0 ? c : -c - 1;
-          Cpx<T> v = stage_sg ? stage[ca] : g.effval_sg ? srcg[(ca >> 2) * 32 + (ca & 3)] : src[ca];
+          Cpx<T> v = stage_sg ? stage[ca] : g.effval_sg ? srcg[sizeof(T) == 8 ? (ca >> 1) * 16 + (ca & 1) : (ca >> 2) * 32 + (ca & 3)] : src[ca];
           if (c < 0) v.im = -v.im;
           y[kz] = v;
         }
@@ -1082,57 +1082,36 @@ __global__ void __launch_bounds__(NTHR) k_m2l_had_tz(const Cpx<T>* __restrict__ 
       done_cnt[b] = 0;
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (NBUF == 2) {
-      bulk_load(smem_addr(Tbuf), ttiles, TILE_BYTES, smem_addr(&bars[0]));
-      if (FTILES > 1) bulk_load(smem_addr(Tbuf + TILE), ttiles + TILE, TILE_BYTES, smem_addr(&bars[1]));
-    }
+    bulk_load(smem_addr(Tbuf), ttiles, TILE_BYTES, smem_addr(&bars[0]));
+    if (FTILES > 1) bulk_load(smem_addr(Tbuf + TILE), ttiles + TILE, TILE_BYTES, smem_addr(&bars[1]));
   }
   __syncthreads();
-  if constexpr (NBUF == 2) {
-    for (int ft = 0; ft < FTILES; ft++) {
-      const int b = ft & 1;
-      const bool ok = mbar_wait_bounded(smem_addr(&bars[b]), (ft >> 1) & 1);
-      if (!ok) {
-        if (lane == 0) atomicOr(status, 1);
-        return;
-      }
-      tz_tile<T, NF, SD, TD>(Tbuf + (size_t)b * TILE, spectra, &claim[b], qend, ft * TZ_F + (lane & 15), qchd, coll,
-                             mask, effval, zero_node, sc, tc, acc != 0);
-      if (lane == 0) {
-        if (atomicAdd(&done_cnt[b], 1) == NW - 1) {  // the last warp out of tile ft
-          done_cnt[b] = 0;
-          claim[b] = qbeg;
-          if (ft + 2 < FTILES)
-            bulk_load(smem_addr(Tbuf + (size_t)b * TILE), ttiles + (size_t)(ft + 2) * TILE, TILE_BYTES,
-                      smem_addr(&bars[b]));
-        }
-      }
-      __syncwarp();
+  for (int ft = 0; ft < FTILES; ft++) {
+    const int b = ft & 1;
+    const bool ok = mbar_wait_bounded(smem_addr(&bars[b]), (ft >> 1) & 1);
+    if (!ok) {
+      if (lane == 0) atomicOr(status, 1);
+      return;
     }
-  } else {
-    for (int ft = 0; ft < FTILES; ft++) {
-      if (threadIdx.x == 0) {
-        claim[0] = qbeg;
-        bulk_load(smem_addr(Tbuf), ttiles + (size_t)ft * TILE, TILE_BYTES, smem_addr(&bars[0]));
+    tz_tile<T, NF, SD, TD>(Tbuf + (size_t)b * TILE, spectra, &claim[b], qend, ft * TZ_F + (lane & 15), qchd, coll,
+                           mask, effval, zero_node, sc, tc, acc != 0);
+    if (lane == 0) {
+      if (atomicAdd(&done_cnt[b], 1) == NW - 1) {  // the last warp out of tile ft
+        done_cnt[b] = 0;
+        claim[b] = qbeg;
+        if (ft + 2 < FTILES)
+          bulk_load(smem_addr(Tbuf + (size_t)b * TILE), ttiles + (size_t)(ft + 2) * TILE, TILE_BYTES,
+                    smem_addr(&bars[b]));
       }
-      __syncthreads();
-      const bool ok = mbar_wait_bounded(smem_addr(&bars[0]), ft & 1);
-      if (__syncthreads_or(!ok)) {
-        if (threadIdx.x == 0) atomicOr(status, 1);
-        return;
-      }
-      tz_tile<T, NF, SD, TD>(Tbuf, spectra, &claim[0], qend, ft * TZ_F + (lane & 15), qchd, coll, mask, effval,
-                             zero_node, sc, tc, acc != 0);
-      __syncthreads();
     }
+    __syncwarp();
   }
 }
 
 template <typename T, int NF, int SD, int TD>
 void tz_launch(const T* ttiles, const T* spectra, int nq, const int* qchd, const int* coll, const unsigned char* mask,
                T* effval, int zero_node, int* status, int num_sms, cudaStream_t st) {
-  constexpr int NTHR = sizeof(T) == 4 ? 512 : 256;
-  constexpr int NBUF = sizeof(T) == 4 ? 2 : 1;
+  constexpr int NTHR = 512, NBUF = 2;
   const size_t smem = (size_t)NBUF * TZ_ROWS * TZ_F * sizeof(Cpx<T>);
   auto kern = k_m2l_had_tz<T, NF, NTHR, NBUF, SD, TD>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1210,24 +1189,21 @@ void launch_m2l_hadamard_sweep(int nf, int sd, int td, const T* ktiles, const T*
     sweep_dofs<T, 2052>(sd, td, ktiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
 }
 
-template <typename T>
-void launch_m2l_hadamard_tz(int nf, int sd, int td, const T* ttiles, const T* spectra, int nq, const int* qchd,
-                            const int* coll, const unsigned char* mask, T* effval, int zero_node, int* status,
+void launch_m2l_hadamard_tz(int nf, int sd, int td, const float* ttiles, const float* spectra, int nq, const int* qchd,
+                            const int* coll, const unsigned char* mask, float* effval, int zero_node, int* status,
                             int num_sms, cudaStream_t st) {
   if (nq <= 0) return;
   if (nf == 868)
-    tz_dofs<T, 868>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_dofs<float, 868>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
   else if (nf == 260)
-    tz_dofs<T, 260>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_dofs<float, 260>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
   else if (nf == 2052)
-    tz_dofs<T, 2052>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_dofs<float, 2052>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
 }
 
 #define KIFMM_INST(T)                                                                                             \
   template void launch_m2l_hadamard_sweep<T>(int, int, int, const T*, const T*, int, const int*, const int*,     \
                                              const unsigned char*, T*, int, int*, int, cudaStream_t);              \
-  template void launch_m2l_hadamard_tz<T>(int, int, int, const T*, const T*, int, const int*, const int*,        \
-                                          const unsigned char*, T*, int, int*, int, cudaStream_t);                 \
   template void launch_m2l_forward<T>(const M2LGeom&, const T*, const int*, int, const int*, T*, cudaStream_t);  \
   template void launch_m2l_hadamard<T>(const M2LGeom&, const T*, const T*, const int*, int, const int64_t*,     \
                                        const int*, const int*, T*, cudaStream_t);                                \
