@@ -453,8 +453,10 @@ struct Impl : ImplBase {
         off_up = level_offsets(all_up_lvl, md);
         off_dn = level_offsets(all_dn_lvl, md);
       }
-      gemm_ws_len = (size_t)4 << 20;  // split-K slices of the shallow levels (32 MB)
-      gemm_ws = dalloc<double>(gemm_ws_len);
+      if (sizeof(T) == 4) {
+        gemm_ws_len = (size_t)4 << 20;  // split-K slices of the shallow levels (32 MB)
+        gemm_ws = dalloc<double>(gemm_ws_len);
+      }
     }
     // V list (M2L), forward set
     {
@@ -961,8 +963,11 @@ struct Impl : ImplBase {
         return;
       }
     }
-    nlaunch += launch_node_gemm<T>(A.M, A.K, A.a, B, ldb, bidx, C, ldc, cidx, ncol, acc, s, gemm_ws, gemm_ws_len,
-                                   num_sms, st);
+    if constexpr (sizeof(T) == 8)
+      nlaunch += launch_node_gemm64(A.M, A.K, A.a, B, ldb, bidx, C, ldc, cidx, ncol, acc, s, num_sms, st);
+    else
+      nlaunch += launch_node_gemm(A.M, A.K, A.a, B, ldb, bidx, C, ldc, cidx, ncol, acc, s, gemm_ws, gemm_ws_len,
+                                  num_sms, st);
   }
 
   // a P2P pass for density vector rhs (global index, selects the sorted

@@ -129,9 +129,8 @@ __global__ void k_node_gemm_reduce(int M, int ncol, int nslice, const double* __
 
 }  // namespace
 
-template <typename T>
-int launch_node_gemm(int M, int K, const T* A, const T* B, int64_t ldb, const int* bidx, T* C, int64_t ldc,
-                      const int* cidx, int ncol, bool accumulate, const GemmScale& sc, double* ws, size_t ws_len,
+int launch_node_gemm(int M, int K, const float* A, const float* B, int64_t ldb, const int* bidx, float* C, int64_t ldc,
+                     const int* cidx, int ncol, bool accumulate, const GemmScale& sc, double* ws, size_t ws_len,
                       int num_sms, cudaStream_t st) {
   if (ncol <= 0 || M <= 0 || K <= 0) return 0;
   const int tiles = ((ncol + BN - 1) / BN) * ((M + BM - 1) / BM);
@@ -144,12 +143,12 @@ int launch_node_gemm(int M, int K, const T* A, const T* B, int64_t ldb, const in
   int kchunk = ((K + ks - 1) / ks + BK - 1) / BK * BK;
   ks = (K + kchunk - 1) / kchunk;
   dim3 grid((ncol + BN - 1) / BN, (M + BM - 1) / BM, ks);
-  k_node_gemm<T><<<grid, NTH, 0, st>>>(M, K, kchunk, A, B, ldb, bidx, C, ldc, cidx, ncol, accumulate ? 1 : 0, sc,
+  k_node_gemm<float><<<grid, NTH, 0, st>>>(M, K, kchunk, A, B, ldb, bidx, C, ldc, cidx, ncol, accumulate ? 1 : 0, sc,
                                        ks > 1 ? ws : nullptr);
   if (ks > 1) {
     size_t n = (size_t)ncol * M;
     int g = (int)std::min<size_t>((n + 255) / 256, (size_t)num_sms * 8);
-    k_node_gemm_reduce<T><<<g, 256, 0, st>>>(M, ncol, ks, ws, C, ldc, cidx, accumulate ? 1 : 0, sc);
+    k_node_gemm_reduce<float><<<g, 256, 0, st>>>(M, ncol, ks, ws, C, ldc, cidx, accumulate ? 1 : 0, sc);
   }
   return ks > 1 ? 2 : 1;
 }
@@ -161,12 +160,5 @@ void launch_node_gemm_reduce_f(int M, int ncol, int nslice, const double* partia
   int g = (int)std::min<size_t>((n + 255) / 256, (size_t)num_sms * 8);
   k_node_gemm_reduce<float><<<g, 256, 0, st>>>(M, ncol, nslice, partial, C, ldc, cidx, accumulate ? 1 : 0, sc);
 }
-
-template int launch_node_gemm<double>(int, int, const double*, const double*, int64_t, const int*, double*,
-                                               int64_t, const int*, int, bool, const GemmScale&, double*, size_t, int,
-                                               cudaStream_t);
-template int launch_node_gemm<float>(int, int, const float*, const float*, int64_t, const int*, float*, int64_t,
-                                            const int*, int, bool, const GemmScale&, double*, size_t, int,
-                                            cudaStream_t);
 
 }  // namespace kifmm

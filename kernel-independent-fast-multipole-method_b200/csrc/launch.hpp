@@ -105,12 +105,17 @@ struct GemmScale {
   int lvl_base = 0;
 };
 
-// ws (FP64, ws_len doubles) lets a launch with few columns split K over
-// several CTAs; pass nullptr to disable.
-template <typename T>
-int launch_node_gemm(int M, int K, const T* A, const T* B, int64_t ldb, const int* bidx, T* C, int64_t ldc,
-                      const int* cidx, int ncol, bool accumulate, const GemmScale& sc, double* ws, size_t ws_len,
-                      int num_sms, cudaStream_t st);
+// FP32 (gemm.cu); ws (FP64, ws_len doubles) lets a launch with few columns split
+// K over several CTAs; pass nullptr to disable.  Returns the number of launches.
+int launch_node_gemm(int M, int K, const float* A, const float* B, int64_t ldb, const int* bidx, float* C, int64_t ldc,
+                     const int* cidx, int ncol, bool accumulate, const GemmScale& sc, double* ws, size_t ws_len,
+                     int num_sms, cudaStream_t st);
+// FP64 on the matrix instructions (gemm_f64.cu), one launch.  M, K, ldb and ldc
+// even (every surface has an even number of points, ranks are padded to
+// multiples of 8), A, B and C 16-byte aligned.
+int launch_node_gemm64(int M, int K, const double* A, const double* B, int64_t ldb, const int* bidx, double* C,
+                       int64_t ldc, const int* cidx, int ncol, bool accumulate, const GemmScale& sc, int num_sms,
+                       cudaStream_t st);
 
 // The same product on the tensor cores (tcgen05, kind::tf32) for FP32 data,
 // with both operands split into a TF32 head and a TF32 tail and three MMAs
