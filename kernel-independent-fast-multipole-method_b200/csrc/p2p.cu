@@ -220,36 +220,70 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
   return r;
 }
 
-// sum over the pairs q = sg, sg + nsplit, ... < npairs of w / |t - s| (the
-// 1e-16 cut-off as in keval), for target t = (px, py, pz)
-__device__ __forceinline__ float lap_pairs(const WarpSrc64<float>& w, float px, float py, float pz, int sg,
-                                           int nsplit, int npairs) {
+// s[k] = sum over the pairs q = sg, sg + nsplit, ... < npairs of w / |t_k - s|
+// (the 1e-16 cut-off as in keval), for two targets t_k = (px, py, pz)[k]
+__device__ __forceinline__ void lap_pairs(const WarpSrc64<float>& w, const float* px, const float* py,
+                                          const float* pz, int sg, int nsplit, int npairs, float* s) {
   const float4* wp = reinterpret_cast<const float4*>(w.p);
-  const unsigned long long PX = pk2(px, px), PY = pk2(py, py), PZ = pk2(pz, pz);
-  unsigned long long S = pk2(0.f, 0.f);
+  unsigned long long PX[2], PY[2], PZ[2], S[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    PX[k] = pk2(px[k], px[k]);
+    PY[k] = pk2(py[k], py[k]);
+    PZ[k] = pk2(pz[k], pz[k]);
+    S[k] = pk2(0.f, 0.f);
+  }
   const int rounds = sg < npairs ? (npairs - sg + nsplit - 1) / nsplit : 0;
-#pragma unroll 8
+#pragma unroll 4
   for (int r = 0; r < rounds; r++) {
     const int q = sg + r * nsplit;
     const float4 A = wp[2 * q], B = wp[2 * q + 1];
-    const unsigned long long X = sub2(PX, pk2(A.x, A.y)), Y = sub2(PY, pk2(A.z, A.w)), Z = sub2(PZ, pk2(B.x, B.y));
-    unsigned long long R2 = mul2(X, X);
-    R2 = fma2(Y, Y, R2);
-    R2 = fma2(Z, Z, R2);
-    float r2a, r2b;
-    upk2(R2, r2a, r2b);
-    const float ria = (r2a >= 1e-16f) ? rsqrt_t(r2a) : 0.f, rib = (r2b >= 1e-16f) ? rsqrt_t(r2b) : 0.f;
-    S = fma2(pk2(ria, rib), pk2(B.z, B.w), S);
+    const unsigned long long SX = pk2(A.x, A.y), SY = pk2(A.z, A.w), SZ = pk2(B.x, B.y), SW = pk2(B.z, B.w);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const unsigned long long X = sub2(PX[k], SX), Y = sub2(PY[k], SY), Z = sub2(PZ[k], SZ);
+      unsigned long long R2 = mul2(X, X);
+      R2 = fma2(Y, Y, R2);
+      R2 = fma2(Z, Z, R2);
+      float r2a, r2b;
+      upk2(R2, r2a, r2b);
+      const float ria = (r2a >= 1e-16f) ? rsqrt_t(r2a) : 0.f, rib = (r2b >= 1e-16f) ? rsqrt_t(r2b) : 0.f;
+      S[k] = fma2(pk2(ria, rib), SW, S[k]);
+    }
   }
-  float sa, sb;
-  upk2(S, sa, sb);
-  return sa + sb;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    float sa, sb;
+    upk2(S[k], sa, sb);
+    s[k] = sa + sb;
+  }
 }
 
-// S2M: lane l owns upward check points l, l + 32, ... (R rounds); every
-// staged source (a broadcast load) updates all of them.
+// u_k += c * sum over the sources sg, sg + nsplit, ... (`rounds` of them) of w / |t_k - s|
+template <typename T>
+__device__ __forceinline__ void lap_points(const WarpSrc64<T>& w, const T* px, const T* py, const T* pz, int sg,
+                                           int nsplit, int rounds, T c, T* u0, T* u1) {
+  T s0 = T(0), s1 = T(0);
+#pragma unroll 4
+  for (int r = 0; r < rounds; r++) {
+    const P4<T> s = w.p[sg + r * nsplit];
+    const T x0 = px[0] - s.x, y0 = py[0] - s.y, z0 = pz[0] - s.z;
+    const T x1 = px[1] - s.x, y1 = py[1] - s.y, z1 = pz[1] - s.z;
+    s0 += rinv_cut(x0 * x0 + y0 * y0 + z0 * z0) * s.w;
+    s1 += rinv_cut(x1 * x1 + y1 * y1 + z1 * z1) * s.w;
+  }
+  *u0 += c * s0;
+  *u1 += c * s1;
+}
+
+// S2M: a warp carries R rounds of 32 upward check points of one leaf, of
+// `parts` warps that share its check points; every staged source (a broadcast
+// load) updates all of them.  All R rounds are computed, the last ones on
+// check points past the end where there are any: a test per round keeps
+// the rounds' chains from overlapping.
 template <typename T, int KT, int R>
-__global__ void __launch_bounds__(32 * WP_WARPS) k_s2m_warp(P2PArgs<T> a, const int* work, int nwork, int rhs) {
+__global__ void __launch_bounds__(32 * WP_WARPS)
+    k_s2m_warp(P2PArgs<T> a, const int* work, int nwork, int parts, int rhs) {
   constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD;
   constexpr bool DL = KTraits<KT>::DL;
   __shared__ WarpSrc<T> ws[WP_WARPS];
@@ -257,14 +291,14 @@ __global__ void __launch_bounds__(32 * WP_WARPS) k_s2m_warp(P2PArgs<T> a, const 
   WarpSrc<T>& w = ws[warp];
   const T* den = a.sden + (size_t)rhs * a.ns * SD;
   const int nt = a.nuc;
-  for (int wi = blockIdx.x * WP_WARPS + warp; wi < nwork; wi += gridDim.x * WP_WARPS) {
-    const int g = work[wi];
+  for (int64_t wi = blockIdx.x * WP_WARPS + warp; wi < (int64_t)nwork * parts; wi += gridDim.x * WP_WARPS) {
+    const int g = work[wi / parts], t0 = (int)(wi % parts) * (32 * R) + lane;
     const T rad = (T)a.radius[g];
     const int sb = a.sbeg[g], sc = a.scnt[g];
     T px[R], py[R], pz[R], acc[R][TD];
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      const int ti = lane + 32 * r;
+      const int ti = t0 + 32 * r;
       px[r] = py[r] = pz[r] = T(0);
       if (ti < nt) {
         px[r] = a.uc_unit[3 * ti] * rad;
@@ -329,7 +363,6 @@ __global__ void __launch_bounds__(32 * WP_WARPS) k_s2m_warp(P2PArgs<T> a, const 
                                    SW = pk2(sp.w, sp.w);
 #pragma unroll
           for (int rp = 0; rp < R / 2; rp++) {
-            if (64 * rp >= nt) break;
             const unsigned long long X = sub2(PX[rp], SX), Y = sub2(PY[rp], SY), Z = sub2(PZ[rp], SZ);
             unsigned long long R2 = mul2(X, X);
             R2 = fma2(Y, Y, R2);
@@ -340,16 +373,12 @@ __global__ void __launch_bounds__(32 * WP_WARPS) k_s2m_warp(P2PArgs<T> a, const 
             SP[rp] = fma2(pk2(ria, rib), SW, SP[rp]);
           }
           if constexpr (R % 2 == 1) {
-            if (32 * (R - 1) < nt) {
-              const float x = px[R - 1] - sp.x, y = py[R - 1] - sp.y, z = pz[R - 1] - sp.z;
-              const float r2 = x * x + y * y + z * z;
-              s_last += ((r2 >= 1e-16f) ? rsqrt_t(r2) : 0.f) * sp.w;
-            }
+            const float x = px[R - 1] - sp.x, y = py[R - 1] - sp.y, z = pz[R - 1] - sp.z;
+            s_last += rinv_cut(x * x + y * y + z * z) * sp.w;
           }
         } else {
 #pragma unroll
-          for (int r = 0; r < R; r++)
-            if (32 * r < nt) keval<KT, T>(px[r] - sp.x, py[r] - sp.y, pz[r] - sp.z, nrm, f, acc[r], a.ku);
+          for (int r = 0; r < R; r++) keval<KT, T>(px[r] - sp.x, py[r] - sp.y, pz[r] - sp.z, nrm, f, acc[r], a.ku);
         }
       }
     }
@@ -366,7 +395,7 @@ __global__ void __launch_bounds__(32 * WP_WARPS) k_s2m_warp(P2PArgs<T> a, const 
     T* outbase = a.supcval + (size_t)g * nt * TD;
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      const int ti = lane + 32 * r;
+      const int ti = t0 + 32 * r;
       if (ti < nt)
 #pragma unroll
         for (int d = 0; d < TD; d++) outbase[(size_t)ti * TD + d] = acc[r][d];
@@ -376,10 +405,13 @@ __global__ void __launch_bounds__(32 * WP_WARPS) k_s2m_warp(P2PArgs<T> a, const 
 
 // Leaf pass, one warp per work item: a round of up to 32 targets of one leaf
 // against a range of the leaf's sources (leaf_items below cuts long ranges).
-// lane = (target slot, source split) with G = the power of two >= the round's
-// target count (<= 32) slots and 32 / G splits, so a leaf of 33-64 targets
-// splits its last round's sources over the lanes its few targets leave;
-// splits are summed with warp shuffles.  Sources are staged 64 at a time: point
+// lane = (target slot, source split) with two targets a slot, G = the power of
+// two >= half the round's targets (<= 16) slots and 32 / G splits, so a leaf of
+// 33-64 targets splits its last round's sources over the lanes its few targets
+// leave; splits are summed with warp shuffles.  Two targets, because a staged
+// source costs a lane 32 (FP64) or, for a pair of them, 32 (FP32) bytes of
+// register fills, at 128 bytes a clock per SM 8 clocks a warp, against 6.5 clocks
+// of FP64 pipe or 4 of reciprocal roots for one target's Laplace terms.  Sources are staged 64 at a time: point
 // sources from the leaf's near list (segments = source leaves, found by
 // bisection of the warp's prefix sums), then the W-list upward equivalent
 // surfaces and the leaf's own downward equivalent surface.  An item of a cut
@@ -423,17 +455,20 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const Le
     int left = it.take;  // point sources of this item still to come
     {
       int G = 1;
-      while (G < nt - it.tb && G < 32) G <<= 1;
+      while (2 * G < nt - it.tb && G < 16) G <<= 1;
       const int nsplit = 32 / G, slot = lane % G, sg = lane / G;
-      const int ti = it.tb + slot;
-      const bool valid = ti < nt;
-      T px = 0, py = 0, pz = 0;
-      if (valid) {
-        px = a.tx[tb0 + ti];
-        py = a.ty[tb0 + ti];
-        pz = a.tz[tb0 + ti];
+      bool valid[2];  // targets it.tb + slot and it.tb + slot + G
+      T px[2], py[2], pz[2], acc[2][TD];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int ti = it.tb + slot + k * G;
+        valid[k] = ti < nt;
+        px[k] = valid[k] ? a.tx[tb0 + ti] : T(0);
+        py[k] = valid[k] ? a.ty[tb0 + ti] : T(0);
+        pz[k] = valid[k] ? a.tz[tb0 + ti] : T(0);
+#pragma unroll
+        for (int d = 0; d < TD; d++) acc[k][d] = T(0);
       }
-      T acc[4] = {0, 0, 0, 0};
       // point sources, up to 32 source leaves per batch
       for (int64_t c0 = nb; c0 < ne; c0 += 32) {
         const int nseg = (int)min((int64_t)32, ne - c0);
@@ -494,23 +529,17 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const Le
             }
           }
           __syncwarp();
-          if (valid) {
+          if (valid[0]) {
             const int rounds = sg < cnt ? (cnt - sg + nsplit - 1) / nsplit : 0;
             if constexpr (PAIR_NEAR) {  // sum f / r on source pairs, times 1/(4 pi) once
-              acc[0] += a.ku.c0 * lap_pairs(w, px, py, pz, sg, nsplit, (cnt + 1) >> 1);
+              float s1[2];
+              lap_pairs(w, px, py, pz, sg, nsplit, (cnt + 1) >> 1, s1);
+              acc[0][0] += a.ku.c0 * s1[0];
+              acc[1][0] += a.ku.c0 * s1[1];
             } else if constexpr (KT == 111) {  // FP64: sum f / r, times 1/(4 pi) once
-              T s1 = T(0);
-#pragma unroll 4
-              for (int r = 0; r < rounds; r++) {
-                const P4<T> s = w.p[sg + r * nsplit];
-                const T x = px - s.x, y = py - s.y, z = pz - s.z;
-                const T r2 = x * x + y * y + z * z;
-                const T ri = rinv_cut(r2);
-                s1 += ri * s.w;
-              }
-              acc[0] += a.ku.c0 * s1;
+              lap_points<T>(w, px, py, pz, sg, nsplit, rounds, a.ku.c0, acc[0], acc[1]);
             } else {
-#pragma unroll 4
+#pragma unroll 2
               for (int r = 0; r < rounds; r++) {
                 const int j = sg + r * nsplit;
                 const P4<T> s = w.p[j];
@@ -524,7 +553,8 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const Le
                   nrm[1] = w.n[3 * j + 1];
                   nrm[2] = w.n[3 * j + 2];
                 }
-                keval<KT, T>(px - s.x, py - s.y, pz - s.z, nrm, f, acc, a.ku);
+#pragma unroll
+                for (int k = 0; k < 2; k++) keval<KT, T>(px[k] - s.x, py[k] - s.y, pz[k] - s.z, nrm, f, acc[k], a.ku);
               }
             }
           }
@@ -577,23 +607,17 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const Le
             for (int s = 1; s < SDM; s++) w.f[jl * (SDM - 1) + s - 1] = sd[(size_t)m * SDM + s];
           }
           __syncwarp();
-          if (valid) {
+          if (valid[0]) {
             const int rounds = sg < cnt ? (cnt - sg + nsplit - 1) / nsplit : 0;
             if constexpr (PAIR_SURF) {
-              acc[0] += a.km.c0 * lap_pairs(w, px, py, pz, sg, nsplit, (cnt + 1) >> 1);
+              float s1[2];
+              lap_pairs(w, px, py, pz, sg, nsplit, (cnt + 1) >> 1, s1);
+              acc[0][0] += a.km.c0 * s1[0];
+              acc[1][0] += a.km.c0 * s1[1];
             } else if constexpr (MM == 111) {
-              T s1 = T(0);
-#pragma unroll 4
-              for (int r = 0; r < rounds; r++) {
-                const P4<T> s = w.p[sg + r * nsplit];
-                const T x = px - s.x, y = py - s.y, z = pz - s.z;
-                const T r2 = x * x + y * y + z * z;
-                const T ri = rinv_cut(r2);
-                s1 += ri * s.w;
-              }
-              acc[0] += a.km.c0 * s1;
+              lap_points<T>(w, px, py, pz, sg, nsplit, rounds, a.km.c0, acc[0], acc[1]);
             } else {
-#pragma unroll 4
+#pragma unroll 2
               for (int r = 0; r < rounds; r++) {
                 const int j = sg + r * nsplit;
                 const P4<T> s = w.p[j];
@@ -602,7 +626,8 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const Le
 #pragma unroll
                 for (int k = 1; k < SDM; k++) f[k] = w.f[j * (SDM - 1) + k - 1];
                 T nrm[3];
-                keval<MM, T>(px - s.x, py - s.y, pz - s.z, nrm, f, acc, a.km);
+#pragma unroll
+                for (int k = 0; k < 2; k++) keval<MM, T>(px[k] - s.x, py[k] - s.y, pz[k] - s.z, nrm, f, acc[k], a.km);
               }
             }
           }
@@ -611,13 +636,16 @@ __global__ void __launch_bounds__(32 * NWARP) k_leaf_warp(P2PArgs<T> a, const Le
       }
       // sum the splits (lanes slot, slot + G, ...)
 #pragma unroll
-      for (int d = 0; d < TD; d++)
-        for (int o = G; o < 32; o <<= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
-      if (valid && sg == 0) {
-        T* o = it.out >= 0 ? partial + ((size_t)it.out * 32 + slot) * TD
-                           : a.tval + ((size_t)rhs * a.nt + tb0 + ti) * TD;
+      for (int k = 0; k < 2; k++) {
 #pragma unroll
-        for (int d = 0; d < TD; d++) o[d] = acc[d];
+        for (int d = 0; d < TD; d++)
+          for (int o = G; o < 32; o <<= 1) acc[k][d] += __shfl_xor_sync(0xffffffffu, acc[k][d], o);
+        if (valid[k] && sg == 0) {
+          T* o = it.out >= 0 ? partial + ((size_t)it.out * 32 + slot + k * G) * TD
+                             : a.tval + ((size_t)rhs * a.nt + tb0 + it.tb + slot + k * G) * TD;
+#pragma unroll
+          for (int d = 0; d < TD; d++) o[d] = acc[k][d];
+        }
       }
     }
   }
@@ -679,13 +707,31 @@ void launch_p2p_kt(const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cu
   switch (which) {
     case P2P_S2M:
       if (w.n) {
-        const int grid = std::min((w.n + WP_WARPS - 1) / WP_WARPS, 148 * 32);
-        if (a.nuc <= 160)
-          k_s2m_warp<T, KT, 5><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, rhs);
-        else if (a.nuc <= 320)
-          k_s2m_warp<T, KT, 10><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, rhs);
-        else  // |UC| <= 488 for np <= 8
-          k_s2m_warp<T, KT, 16><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, rhs);
+        // rounds per warp.  FP32: all of a leaf's (152, 296 and 488 check points at
+        // np = 4, 6 and 8 are 5, 10 and 16 rounds).  FP64: 5 or 4 of them, which
+        // reuse a staged source often enough (two would) at half the registers.
+        // Two rounds where the leaves alone leave the SMs below 32 warps, so that
+        // one warp's rounds do not set the time, and for other np.
+        const int rounds = (a.nuc + 31) / 32;
+        int R = 2;
+        if (w.n >= 148 * 32) {
+          if (sizeof(T) == 8)
+            R = rounds % 5 == 0 ? 5 : rounds % 4 == 0 ? 4 : 2;
+          else if (rounds == 5 || rounds == 10 || rounds == 16)
+            R = rounds;
+        }
+        const int parts = (rounds + R - 1) / R;
+        const int grid = (int)std::min<int64_t>(((int64_t)w.n * parts + WP_WARPS - 1) / WP_WARPS, 148 * 32);
+        if (R == 2)
+          k_s2m_warp<T, KT, 2><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+        else if (R == 5)
+          k_s2m_warp<T, KT, 5><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+        else if constexpr (sizeof(T) == 8)
+          k_s2m_warp<T, KT, 4><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+        else if (R == 10)
+          k_s2m_warp<T, KT, 10><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+        else
+          k_s2m_warp<T, KT, 16><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
       }
       break;
     case P2P_S2L:
