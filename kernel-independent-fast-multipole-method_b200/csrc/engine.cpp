@@ -236,7 +236,7 @@ struct Impl : ImplBase {
   std::shared_ptr<Had64Tables> had64_shared;  // ... held from the per-device cache
   Had64Groups had64_grp;                // ... and its groups of target parents
   unsigned* htc_dirs = nullptr;     // tensor-core Hadamard: directions present per tile of 128 parents
-  int* h_status = nullptr;  // mapped host word: device-side wait time-outs (bit 0 sweep, bit 1 GEMM, bit 2 TC Hadamard)
+  int* h_status = nullptr;  // mapped host word: device-side wait time-outs (bit 0 sweeps, bit 1 GEMM, bits 2 and 3 the tensor-core Hadamard)
   int* d_status = nullptr;
   List s2m, s2l, leaf, m2l, fwd;
   std::vector<List> up_non, dn_par;
@@ -453,7 +453,7 @@ struct Impl : ImplBase {
         off_up = level_offsets(all_up_lvl, md);
         off_dn = level_offsets(all_dn_lvl, md);
       }
-      if (sizeof(T) == 4) {
+      if (sizeof(T) == 4 && !use_tc) {
         gemm_ws_len = (size_t)4 << 20;  // split-K slices of the shallow levels (32 MB)
         gemm_ws = dalloc<double>(gemm_ws_len);
       }
@@ -958,8 +958,8 @@ struct Impl : ImplBase {
     s.lvl_base = E.rootlvl;
     if constexpr (sizeof(T) == 4) {
       if (A.tc.img && ldb % 4 == 0 && ldc % 4 == 0) {
-        nlaunch += launch_node_gemm_tc(A.tc, B, ldb, bidx, C, ldc, cidx, ncol, acc, s, gemm_ws, gemm_ws_len, num_sms,
-                                       d_status, st);
+        nlaunch += launch_node_gemm_tc(A.tc, B, ldb, bidx, C, ldc, cidx, ncol, acc, s, num_sms, d_status,
+                                       st);
         return;
       }
     }

@@ -138,7 +138,7 @@ __device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigne
                : "memory");
 }
 
-// Work items are (node tile, N tile, K split); the grid is persistent (at
+// Work items are (node tile, N tile); the grid is persistent (at
 // most one CTA per SM, each looping over items blockIdx.x, + gridDim.x, ...).
 // Warp-specialised: warps 0-7 stage node data (A stages, two) and drain the
 // accumulators (two), warp 8 issues the MMAs and the operator bulk copies (B
@@ -155,28 +155,22 @@ constexpr int TC_ALL = TC_WORKERS + 32;
 __global__ void __launch_bounds__(TC_ALL, 1) k_node_gemm_tc(TcOperator A, const float* __restrict__ B, int64_t ldb,
                                                            const int* __restrict__ bidx, float* __restrict__ C,
                                                            int64_t ldc, const int* __restrict__ cidx, int ncol,
-                                                           int accumulate, GemmScale sc, int kper, int nitems,
-                                                           double* __restrict__ partial, int* __restrict__ status) {
+                                                           int accumulate, GemmScale sc, int nitems,
+                                                           int* __restrict__ status) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) unsigned long long afull[2], bfull[3], accfull[2], accempty[2];
   __shared__ unsigned tmem_base;
   __shared__ int fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int gx = (ncol + TC_M - 1) / TC_M, gy = A.ntiles;
-  const int nkt = A.Kp / TC_KC;
+  const int gx = (ncol + TC_M - 1) / TC_M;
   if ((int)blockIdx.x >= nitems) return;
   const int my_items = (nitems - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
-  auto item_of = [&](int li, int& x, int& y, int& z) {
+  auto item_of = [&](int li, int& x, int& y) {
     const int it = blockIdx.x + li * gridDim.x;
     x = it % gx;
-    y = (it / gx) % gy;
-    z = it / (gx * gy);
+    y = it / gx;
   };
-  int x0, y0, z0;
-  item_of(0, x0, y0, z0);
-  // every item of one launch has the same chunk count except a shorter last K
-  // split, which only split launches (one item per CTA) have
-  const int nk = min(nkt, (z0 + 1) * kper) - z0 * kper;
+  const int nk = A.Kp / TC_KC;  // chunks per item
   const int total = my_items * nk;
 
   if (warp == 0) {
@@ -202,8 +196,8 @@ __global__ void __launch_bounds__(TC_ALL, 1) k_node_gemm_tc(TcOperator A, const 
   auto a_stage = [&](int g) { return smem + (g & 1) * A_STAGE; };
   auto b_stage = [&](int g) { return smem + 2 * A_STAGE + (g % 3) * B_STAGE; };
   auto half_of = [&](int g) {
-    int x, y, z;
-    item_of(g / nk, x, y, z);
+    int x, y;
+    item_of(g / nk, x, y);
     return min(A.ntile, A.Np - y * A.ntile) / 2;
   };
   volatile int* vfail = &fail;
@@ -221,9 +215,9 @@ __global__ void __launch_bounds__(TC_ALL, 1) k_node_gemm_tc(TcOperator A, const 
     {
       auto issue_op = [&](int g) {
         if (g >= total || lane != 0) return;
-        int x, y, z;
-        item_of(g / nk, x, y, z);
-        const float* img = A.img + ((size_t)y * nkt + z * kper + g % nk) * IMG_FLOATS;
+        int x, y;
+        item_of(g / nk, x, y);
+        const float* img = A.img + ((size_t)y * nk + g % nk) * IMG_FLOATS;
         bulk_load(smem_u32(b_stage(g)), img, IMG_FLOATS * 4, smem_u32(&bfull[g % 3]));
       };
       issue_op(0);
@@ -260,8 +254,8 @@ __global__ void __launch_bounds__(TC_ALL, 1) k_node_gemm_tc(TcOperator A, const 
     const int lrow = tid & (TC_M - 1), lq0 = (tid >> 7) * 4;
     // node column of this thread's row in item li (-1: past the last node)
     auto item_col = [&](int li) {
-      int x, y, z;
-      item_of(li, x, y, z);
+      int x, y;
+      item_of(li, x, y);
       const int lj = x * TC_M + lrow;
       return lj < ncol ? bidx[lj] : -1;
     };
@@ -279,9 +273,9 @@ __global__ void __launch_bounds__(TC_ALL, 1) k_node_gemm_tc(TcOperator A, const 
           li_cur = li;
           idx_next = li + 1 < my_items ? item_col(li + 1) : -1;
         }
-        int x, y, z;
-        item_of(li, x, y, z);
-        k0 = (z * kper + g % nk) * TC_KC;
+        int x, y;
+        item_of(li, x, y);
+        k0 = g % nk * TC_KC;
         have = bcol != nullptr;
       }
 #pragma unroll
@@ -333,17 +327,12 @@ __global__ void __launch_bounds__(TC_ALL, 1) k_node_gemm_tc(TcOperator A, const 
     };
     // store item li's tile from the sums (row (warp & 3) * 32 + lane, this thread's half)
     auto epilogue = [&](int li) {
-      int x, y, z;
-      item_of(li, x, y, z);
+      int x, y;
+      item_of(li, x, y);
       const int n0 = y * A.ntile, nn = min(A.ntile, A.Np - n0), half = nn / 2;
       const int j = x * TC_M + (warp & 3) * 32 + lane;
       const int nb = n0 + (warp >> 2) * half;
-      if (j < ncol && partial) {  // split K: raw sums, scaled and added by the reduce
-        double* pr = partial + ((size_t)z * ncol + j) * A.M;
-#pragma unroll
-        for (int i = 0; i < TC_HALF; i++)
-          if (i < half && nb + i < A.M) pr[nb + i] = (double)sum[i];
-      } else if (j < ncol) {
+      if (j < ncol) {
         float* crow = C + (int64_t)cidx[j] * ldc;
         const int lvl = sc.col_lvl ? sc.col_lvl[j] + sc.lvl_base : 0;
         float f4[4];  // scale of output n: f4[n % sd], sd <= 4
@@ -442,29 +431,16 @@ void tc_operator_images(int M, int K, const double* A, std::vector<float>* img, 
 }
 
 int launch_node_gemm_tc(const TcOperator& A, const float* B, int64_t ldb, const int* bidx, float* C, int64_t ldc,
-                        const int* cidx, int ncol, bool accumulate, const GemmScale& sc, double* ws, size_t ws_len,
-                        int num_sms, int* status, cudaStream_t st) {
+                        const int* cidx, int ncol, bool accumulate, const GemmScale& sc, int num_sms, int* status,
+                        cudaStream_t st) {
   if (ncol <= 0 || A.M <= 0 || A.K <= 0) return 0;
-  const int gx = (ncol + TC_M - 1) / TC_M, gy = A.ntiles;
-  const int nk = A.Kp / TC_KC;
-  // few tiles (the shallow tree levels): split K so that every SM has work
-  int splits = 1;
-  if (ws && gx * gy < num_sms && nk >= 4) {
-    splits = std::min({(2 * num_sms) / (gx * gy), nk / 2, 16});
-    while (splits > 1 && (size_t)splits * ncol * A.M > ws_len) splits--;
-    splits = std::max(splits, 1);
-  }
-  const int kper = (nk + splits - 1) / splits;
-  splits = (nk + kper - 1) / kper;
-  const int nitems = gx * gy * splits;
-  // split launches: one item per CTA (the last split may be shorter);
-  // otherwise persistent, at most one CTA per SM
-  const int grid = splits > 1 ? nitems : std::min(nitems, num_sms);
+  const int nitems = (ncol + TC_M - 1) / TC_M * A.ntiles;
+  if (nitems < num_sms)  // a level's few tiles: smaller tiles, K split over clusters
+    return launch_node_gemm_tf32(A, B, ldb, bidx, C, ldc, cidx, ncol, accumulate, sc, num_sms, st);
   cudaFuncSetAttribute(k_node_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
-  k_node_gemm_tc<<<grid, TC_ALL, TC_SMEM, st>>>(A, B, ldb, bidx, C, ldc, cidx, ncol, accumulate ? 1 : 0, sc, kper,
-                                                 nitems, splits > 1 ? ws : nullptr, status);
-  if (splits > 1) launch_node_gemm_reduce_f(A.M, ncol, splits, ws, C, ldc, cidx, accumulate, sc, num_sms, st);
-  return splits > 1 ? 2 : 1;
+  k_node_gemm_tc<<<std::min(nitems, num_sms), TC_ALL, TC_SMEM, st>>>(A, B, ldb, bidx, C, ldc, cidx, ncol,
+                                                                     accumulate ? 1 : 0, sc, nitems, status);
+  return 1;
 }
 
 }  // namespace kifmm

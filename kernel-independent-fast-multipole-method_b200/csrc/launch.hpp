@@ -117,33 +117,30 @@ int launch_node_gemm64(int M, int K, const double* A, const double* B, int64_t l
                        int64_t ldc, const int* cidx, int ncol, bool accumulate, const GemmScale& sc, int num_sms,
                        cudaStream_t st);
 
-// The same product on the tensor cores (tcgen05, kind::tf32) for FP32 data,
-// with both operands split into a TF32 head and a TF32 tail and three MMAs
-// (head*head + head*tail + tail*head) accumulating in FP32: about 2^-21
-// relative per product, the FP32 rounding class.  The operator is split on
-// the host into shared-memory images, one per (N tile, 32-wide K chunk):
-// head then tail, each 160 rows x 32 columns in the no-swizzle K-major
-// core-matrix layout (zero padded), so that one bulk copy moves a chunk.
-// Requires K, ldb, ldc multiples of 4 and 16-byte aligned B and C.  Launches
-// with fewer tiles than SMs split K over CTAs into ws (FP64, ws_len doubles)
-// and reduce it deterministically.  A bounded wait that times out sets bit 1
-// of *status.  Returns the number of launches.
+// The same product on the tensor cores for FP32 data, both operands split into
+// a TF32 head and a TF32 tail and three MMAs per product (head*head + head*tail +
+// tail*head) accumulating in FP32: about 2^-21 relative, the FP32 rounding
+// class.  The operator is split on the host into shared-memory images, one per
+// (N tile, 32-wide K chunk): head then tail, each 160 rows x 32 columns in the
+// no-swizzle K-major core-matrix layout (zero padded), so that one bulk copy moves
+// a chunk.  Requires M, K, ldb and ldc multiples of 4 and 16-byte aligned B and C.
+// Launches with at least as many tiles of 128 nodes as SMs run on tcgen05
+// (gemm_tc.cu, kind::tf32; a bounded wait that times out sets bit 1 of *status), the
+// others on mma.sync with K split over clusters (gemm_tf32.cu).  One launch.
 struct TcOperator {
   const float* img = nullptr;  // [ntiles][Kp/32][2][160 x 32]
   int M = 0, K = 0, Np = 0, Kp = 0;
   int ntile = 0, ntiles = 0;  // rows per N tile (multiple of 16, <= 160), number of N tiles
 };
 int launch_node_gemm_tc(const TcOperator& A, const float* B, int64_t ldb, const int* bidx, float* C, int64_t ldc,
-                        const int* cidx, int ncol, bool accumulate, const GemmScale& sc, double* ws, size_t ws_len,
-                        int num_sms, int* status, cudaStream_t st);
+                        const int* cidx, int ncol, bool accumulate, const GemmScale& sc, int num_sms, int* status,
+                        cudaStream_t st);
+int launch_node_gemm_tf32(const TcOperator& A, const float* B, int64_t ldb, const int* bidx, float* C, int64_t ldc,
+                          const int* cidx, int ncol, bool accumulate, const GemmScale& sc, int num_sms,
+                          cudaStream_t st);
 // host side: the images of a row-major M x K operator (fills A's sizes; img
 // is left to the caller to upload)
 void tc_operator_images(int M, int K, const double* A, std::vector<float>* img, TcOperator* desc);
-// C[cidx[j]] (=|+=) scaled sum over nslice of partial[z][j][0..M) (gemm.cu)
-void launch_node_gemm_reduce_f(int M, int ncol, int nslice, const double* partial, float* C, int64_t ldc,
-                               const int* cidx, bool accumulate, const GemmScale& sc, int num_sms, cudaStream_t st);
-// host-side split of a row-major M x K operator into the padded hi/lo pair
-void split_tf32(int M, int K, const double* A, std::vector<float>* hi, std::vector<float>* lo, int* Np, int* Kp);
 
 // FFT-based M2L (MatMgnt3d::plnden2effden / UE2DC_dgemv / effval2plnval,
 // fmm3d/matmgnt3d.cpp:223-361).
