@@ -24,6 +24,7 @@
 #include <tuple>
 
 #include "../../include/kifmm.h"
+#include "arena.hpp"
 #include "launch.hpp"
 
 namespace kifmm {
@@ -135,14 +136,12 @@ struct Impl : ImplBase {
   Engine& E;
   const Tree& tr;
   const Operators& op;
-  std::vector<void*> allocs;
+  DeviceArena arena;
 
   template <class U>
   U* dalloc(size_t n) {
     void* p = nullptr;
-    if (n == 0) n = 1;
-    KCHECK(cudaMalloc(&p, n * sizeof(U)));
-    allocs.push_back(p);
+    KCHECK(arena.get(n * sizeof(U), &p));
     return (U*)p;
   }
   template <class U>
@@ -250,7 +249,6 @@ struct Impl : ImplBase {
 
   Impl(Engine& e) : E(e), tr(e.tree), op(*e.ops) {}
   ~Impl() override {
-    for (void* p : allocs) cudaFree(p);
     if (h_status) cudaFreeHost(h_status);
     if (have_events)
       for (auto& x : ev) cudaEventDestroy(x);
@@ -930,6 +928,7 @@ struct Impl : ImplBase {
     replicate(dn_all, R);
     for (auto& L : up_non) replicate(L, R);
     for (auto& L : dn_par) replicate(L, R);
+    KCHECK(cudaStreamSynchronize(0));  // the caller's stream need not wait for the default stream
     cap_chunk = R;
   }
 

@@ -41,6 +41,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "host_parallel.hpp"
 #include "launch.hpp"
 
 namespace kifmm {
@@ -244,19 +245,19 @@ void launch_had64_tables(const double* khat, int nf, int sd, int td, double* tab
 void had64_groups(int nq, int zero_node, const int* qchd, const int* coll, Had64HostGroups* o) {
   constexpr int WINDOW = 1024;
   std::vector<unsigned> dirs(nq, 0u);
-  std::vector<int> order;
-  order.reserve(nq);
-  for (int w = 0; w < nq; w++)
-    for (int d = 0; d < 26; d++)
-      if (coll[(size_t)w * 26 + d] != zero_node) dirs[w] |= 1u << d;
-  std::vector<int> left;
-  for (int b = 0; b < nq; b += WINDOW) {
-    left.clear();
-    for (int w = b; w < std::min(nq, b + WINDOW); w++) left.push_back(w);
+  std::vector<int> order(nq);
+  auto window = [&](int b) {
+    std::vector<int> left;
+    int n = b;
+    for (int w = b; w < std::min(nq, b + WINDOW); w++) {
+      left.push_back(w);
+      for (int d = 0; d < 26; d++)
+        if (coll[(size_t)w * 26 + d] != zero_node) dirs[w] |= 1u << d;
+    }
     while (!left.empty()) {
       // a tile begins with the next parent of the Morton order
       unsigned m = dirs[left[0]];
-      order.push_back(left[0]);
+      order[n++] = left[0];
       left.erase(left.begin());
       for (int k = 1; k < 8 && !left.empty(); k++) {
         int best = 0, cost = 1 << 30;
@@ -269,11 +270,15 @@ void had64_groups(int nq, int zero_node, const int* qchd, const int* coll, Had64
           }
         }
         m |= dirs[left[best]];
-        order.push_back(left[best]);
+        order[n++] = left[best];
         left.erase(left.begin() + best);
       }
     }
-  }
+  };
+  const int windows = (nq + WINDOW - 1) / WINDOW;
+  host_parallel(host_parallel_threads(windows), [&](int t, int n) {
+    for (int k = t; k < windows; k += n) window(k * WINDOW);
+  });
   const int ng = (nq + H_GROUP - 1) / H_GROUP, zero = (zero_node + 7) >> 3;
   o->head.clear();
   o->tab.clear();

@@ -12,6 +12,7 @@
 // Positions are stored relative to the centre of their leaf and re-centred on
 // the target node's centre while staging, so FP32 differences lose no more
 // than the node size's precision.
+#include "host_parallel.hpp"
 #include "kernels_common.cuh"
 #include "launch.hpp"
 
@@ -755,38 +756,14 @@ void launch_p2p_kt(const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cu
 
 }  // namespace
 
-// Work items of the leaf pass.  One warp per leaf, the form before, left a
-// leaf with long lists to one warp (150,001 sources on an ellipsoid, targets
-// in the volume: the coarse leaves' W lists hold hundreds of surfaces, 17.9 ms
-// in that warp's tail) and a small tree's leaves on a few SMs (2,000 points:
-// 56 warps, 0.15 ms).  A range costs its sources over the lanes that share a
-// target; it is cut above `limit` = 1/8 of a warp's share when every SM holds
-// 32 warps, and not below `least` sources (two staged batches in FP64, four in
-// FP32, whose pairs take a quarter of the time), where starting an item and
-// adding its partial sum would cost more than the sources.
-void leaf_items(int nwork, const int* work, const int* tcnt, const int* scnt, const int64_t* nptr, const int* nidx,
-                const int64_t* mptr, const unsigned char* l2t, const int* tbeg, int nsurf, int least, int num_sms,
-                std::vector<LeafItem>* items, std::vector<LeafSplit>* splits, int* nparts) {
-  items->clear();
-  splits->clear();
-  *nparts = 0;
-  auto lanes = [](int left) {  // lanes that share a target in a round with `left` targets to go
-    int G = 1;
-    while (G < left && G < 32) G <<= 1;
-    return 32 / G;
-  };
-  std::vector<int64_t> nsrc(nwork);
-  double total = 0;
-  for (int w = 0; w < nwork; w++) {
-    int64_t s = 0;
-    for (int64_t k = nptr[w]; k < nptr[w + 1]; k++) s += scnt[nidx[k]];
-    nsrc[w] = s;
-    const int nt = tcnt[work[w]];
-    const double all = (double)s + (double)nsurf * ((mptr[w + 1] - mptr[w]) + l2t[w]);
-    for (int tb = 0; tb < nt; tb += 32) total += all / lanes(nt - tb);
-  }
-  const double limit = std::max((double)least, total / ((double)num_sms * 32 * 8));
-  for (int w = 0; w < nwork; w++) {
+namespace {
+// the items of leaves w0 .. w1 - 1 of leaf_items, partial rows counted from 0
+template <class Lanes>
+void cut_leaves(int w0, int w1, const int* work, const int* tcnt, const int* scnt, const int64_t* nptr, const int* nidx,
+                const int64_t* mptr, const unsigned char* l2t, const int* tbeg, int nsurf, double limit,
+                const int64_t* nsrc, Lanes lanes, std::vector<LeafItem>* items, std::vector<LeafSplit>* splits,
+                int* nparts) {
+  for (int w = w0; w < w1; w++) {
     const int g = work[w], nt = tcnt[g];
     const int nseg = (int)(mptr[w + 1] - mptr[w]) + l2t[w];
     const int64_t all = nsrc[w] + (int64_t)nseg * nsurf;
@@ -844,6 +821,71 @@ void leaf_items(int nwork, const int* work, const int* tcnt, const int* scnt, co
         }
       }
     }
+  }
+}
+}  // namespace
+
+// Work items of the leaf pass.  One warp per leaf, the form before, left a
+// leaf with long lists to one warp (150,001 sources on an ellipsoid, targets
+// in the volume: the coarse leaves' W lists hold hundreds of surfaces, 17.9 ms
+// in that warp's tail) and a small tree's leaves on a few SMs (2,000 points:
+// 56 warps, 0.15 ms).  A range costs its sources over the lanes that share a
+// target; it is cut above `limit` = 1/8 of a warp's share when every SM holds
+// 32 warps, and not below `least` sources (two staged batches in FP64, four in
+// FP32, whose pairs take a quarter of the time), where starting an item and
+// adding its partial sum would cost more than the sources.
+void leaf_items(int nwork, const int* work, const int* tcnt, const int* scnt, const int64_t* nptr, const int* nidx,
+                const int64_t* mptr, const unsigned char* l2t, const int* tbeg, int nsurf, int least, int num_sms,
+                std::vector<LeafItem>* items, std::vector<LeafSplit>* splits, int* nparts) {
+  auto lanes = [](int left) {  // lanes that share a target in a round with `left` targets to go
+    int G = 1;
+    while (G < left && G < 32) G <<= 1;
+    return 32 / G;
+  };
+  // the leaves in contiguous ranges, one host thread each
+  const int nthr = host_parallel_threads(nwork / 2048);
+  auto run = [&](auto&& body) {  // body(t, first leaf, past the last)
+    host_parallel(nthr, [&](int t, int n) {
+      body(t, (int)((int64_t)nwork * t / n), (int)((int64_t)nwork * (t + 1) / n));
+    });
+  };
+  std::vector<int64_t> nsrc(nwork);
+  std::vector<double> totals(nthr, 0.0);
+  run([&](int t, int w0, int w1) {
+    double total = 0;
+    for (int w = w0; w < w1; w++) {
+      int64_t s = 0;
+      for (int64_t k = nptr[w]; k < nptr[w + 1]; k++) s += scnt[nidx[k]];
+      nsrc[w] = s;
+      const int nt = tcnt[work[w]];
+      const double all = (double)s + (double)nsurf * ((mptr[w + 1] - mptr[w]) + l2t[w]);
+      for (int tb = 0; tb < nt; tb += 32) total += all / lanes(nt - tb);
+    }
+    totals[t] = total;
+  });
+  double total = 0;
+  for (double v : totals) total += v;
+  const double limit = std::max((double)least, total / ((double)num_sms * 32 * 8));
+  std::vector<std::vector<LeafItem>> pitems(nthr);
+  std::vector<std::vector<LeafSplit>> psplits(nthr);
+  std::vector<int> pparts(nthr, 0);
+  run([&](int t, int w0, int w1) {
+    cut_leaves(w0, w1, work, tcnt, scnt, nptr, nidx, mptr, l2t, tbeg, nsurf, limit, nsrc.data(), lanes, &pitems[t],
+               &psplits[t], &pparts[t]);
+  });
+  items->clear();
+  splits->clear();
+  *nparts = 0;
+  for (int t = 0; t < nthr; t++) {
+    for (LeafItem& it : pitems[t]) {
+      if (it.out >= 0) it.out += *nparts;
+      items->push_back(it);
+    }
+    for (LeafSplit& sp : psplits[t]) {
+      sp.first += *nparts;
+      splits->push_back(sp);
+    }
+    *nparts += pparts[t];
   }
 }
 

@@ -34,6 +34,7 @@
 #include <string>
 #include <vector>
 
+#include "arena.hpp"
 #include "tree.hpp"
 
 namespace kifmm {
@@ -408,10 +409,9 @@ __global__ void k_sort_segments(const long long* __restrict__ ptr, int* __restri
 }
 
 template <class T>
-T* dnew(size_t n, std::vector<void*>& owned) {
+T* dnew(size_t n, DeviceArena& owned) {
   void* p = nullptr;
-  TCHECK(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
-  owned.push_back(p);
+  TCHECK(owned.get(n * sizeof(T), &p));
   return (T*)p;
 }
 
@@ -428,7 +428,7 @@ int build_tree_device(Tree& t, int ns, const double* srcpos, int nt, const doubl
     if (err) *err = "bad ptsmax/maxlevel (maxlevel must be in [1,21])";
     return 1;
   }
-  std::vector<void*> owned;
+  DeviceArena owned;  // freed on return, after the stream has been synchronised
   cudaStream_t st = nullptr;
   int rc = 0;
   try {
@@ -541,7 +541,7 @@ int build_tree_device(Tree& t, int ns, const double* srcpos, int nt, const doubl
     // ---- lists: count, scan, fill, sort
     ListOut lo{};
     for (int l = 0; l < 4; l++) lo.cnt[l] = dnew<int>(nn, owned);
-    k_lists<false><<<(nn + 127) / 128, 128, 0, st>>>(nd, tag, nn, lo);
+    k_lists<false><<<(nn + 31) / 32, 32, 0, st>>>(nd, tag, nn, lo);
     long long* ptr[4];
     for (int l = 0; l < 4; l++) {
       ptr[l] = dnew<long long>((size_t)nn + 1, owned);
@@ -554,7 +554,7 @@ int build_tree_device(Tree& t, int ns, const double* srcpos, int nt, const doubl
       lo.ptr[l] = ptr[l];
       lo.idx[l] = dnew<int>((size_t)tot[l], owned);
     }
-    k_lists<true><<<(nn + 127) / 128, 128, 0, st>>>(nd, tag, nn, lo);
+    k_lists<true><<<(nn + 31) / 32, 32, 0, st>>>(nd, tag, nn, lo);
     // U (descent leaves, then the sorted coarser nodes and the node itself)
     // and W (descent nodes) need sorting; V and X are written sorted
     k_sort_segments<<<(nn + 127) / 128, 128, 0, st>>>(ptr[0], lo.idx[0], nn);
@@ -592,7 +592,6 @@ int build_tree_device(Tree& t, int ns, const double* srcpos, int nt, const doubl
     rc = code;
   }
   if (st) cudaStreamSynchronize(st);
-  for (void* p : owned) cudaFree(p);
   if (st) cudaStreamDestroy(st);
   return rc;
 }
