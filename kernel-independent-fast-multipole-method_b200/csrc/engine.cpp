@@ -50,7 +50,7 @@ struct CudaError {
 // The FP16 operator images of the tensor-core Hadamard on one device, shared
 // by every engine whose translation operators are the same object (the
 // operator cache hands one object per kernel and np to every engine): the
-// images of a multi-dof kernel reach hundreds of MB (Stokes np=6: 217 chunks
+// images of a multi-dof kernel reach hundreds of MB (Stokes np=6: 167 chunks
 // x 26 directions x 12 dof pairs x 4 KB), so instances of a batch keep one
 // copy.  Freed with the last engine that holds them.
 struct Tc16Images {

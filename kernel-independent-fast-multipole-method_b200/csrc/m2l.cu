@@ -2,20 +2,22 @@
 // (fmm3d/fmm3d_eval.cpp:115-150; MatMgnt3d::plnden2effden, UE2DC_dgemv,
 // effval2plnval, fmm3d/matmgnt3d.cpp:223-361).
 //
-// The surface density of a node is a sparse (2np)^3 grid: only the np^3
-// corner block holds data, and only on its boundary.  Instead of a general
+// The surface density of a node is a sparse n^3 grid, n = 2 np - 1 (np source
+// and np target points per axis have 2 np - 1 lags, so this is the smallest
+// cyclic size without wrap-around; the reference's 2 np holds 18 to 34 % more
+// frequencies): only the np^3 corner block holds data, and only on its boundary.  Instead of a general
 // FFT library the transforms are pruned separable DFTs done in shared
 // memory, one CTA per node:
-//   forward : x pass (np^2 lines, np inputs -> np+1 outputs), y pass, z pass
+//   forward : x pass (np^2 lines, np inputs -> np outputs), y pass, z pass
 //   inverse : z and y passes evaluated only at the np outputs the surface
 //             needs, then the Hermitian half-line c2r along x at the surface
 //             points only.
 // The kernel spectra are computed once on the host (operators.cpp) with the
 // same sign convention w = exp(-2 pi i / n) and already carry 1/n^3.
-// Spectra are stored Hermitian-compacted: of the kx = 0 and kx = n/2 planes,
-// which a real grid's half spectrum repeats as X(kx,-ky,-kz) = conj X(kx,ky,kz),
-// only the canonical half is kept (4 np^3 + 4 values instead of 4 np^2 (np+1);
-// 868 of 1008 at np = 6).  The products K X keep the symmetry, so the
+// Spectra are stored Hermitian-compacted: of the kx = 0 plane, which a real
+// grid's half spectrum repeats as X(0,-ky,-kz) = conj X(0,ky,kz), only the
+// canonical half is kept ((n^3 + 1) / 2 values, up to a multiple of 4; 668 at
+// np = 6).  The products K X keep the symmetry, so the
 // forward pass computes, the Hadamard pass multiplies and the inverse pass
 // reads back (conjugating the mirrored half) only the independent values.
 // Density and potential grids use indices [0, np) per axis; the reference's
@@ -76,7 +78,8 @@ __host__ __device__ inline size_t inv_rb_warp_bytes(int np, int n, int nh) {
 // the staged accumulated spectrum of one node (sibling-group-major FP32 form)
 template <typename T>
 __host__ __device__ inline size_t inv_rb_stage_bytes(int np) {
-  return align16(sizeof(Cpx<T>) * (4 * np * np * np + 4));
+  const int n = 2 * np - 1;
+  return align16(sizeof(Cpx<T>) * (((n * n * n + 1) / 2 + 3) / 4 * 4));
 }
 
 template <typename T>
@@ -85,15 +88,14 @@ __host__ __device__ inline size_t inv_warp_bytes(int np, int n, int nh) {
          align16(sizeof(Cpx<T>) * np * np * nh);
 }
 
-template <typename T, int NP>
+template <typename T>
 __global__ void __launch_bounds__(256) k_m2l_fwd_warp(M2LGeom g, const T* __restrict__ supeden,
                                                       const int* __restrict__ nodes, int nwork,
                                                       const int* __restrict__ depth, T* __restrict__ spectra) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // NP > 0: compile-time sizes (constant divisors, unrolled sums); NP = 0: any np
-  const int np = NP > 0 ? NP : g.np, n = NP > 0 ? 2 * NP : g.n, nh = NP > 0 ? NP + 1 : g.nh;
-  const int nfc = NP > 0 ? 4 * NP * NP * NP + 4 : g.nfc;
-  const int nsurf = NP > 0 ? NP * NP * NP - (NP - 2) * (NP - 2) * (NP - 2) : g.nsurf;
+  const int np = g.np, n = g.n, nh = g.nh;
+  const int nfc = g.nfc;
+  const int nsurf = g.nsurf;
   Cpx<T>* W2 = reinterpret_cast<Cpx<T>*>(smem_raw);
   fill_w2(W2, n);
   __syncthreads();
@@ -163,16 +165,15 @@ __global__ void __launch_bounds__(256) k_m2l_fwd_warp(M2LGeom g, const T* __rest
   }
 }
 
-template <typename T, int NP>
+template <typename T>
 __global__ void __launch_bounds__(256) k_m2l_inv_warp(M2LGeom g, const T* __restrict__ effval,
                                                       const int* __restrict__ work, int nwork,
                                                       T* __restrict__ tdncval) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // NP > 0: compile-time sizes (constant divisors, unrolled sums); NP = 0: any np
-  const int np = NP > 0 ? NP : g.np, n = NP > 0 ? 2 * NP : g.n, nh = NP > 0 ? NP + 1 : g.nh;
-  const int nf = NP > 0 ? 4 * NP * NP * (NP + 1) : g.nfreq;
-  const int nfc = NP > 0 ? 4 * NP * NP * NP + 4 : g.nfc;
-  const int nsurf = NP > 0 ? NP * NP * NP - (NP - 2) * (NP - 2) * (NP - 2) : g.nsurf;
+  const int np = g.np, n = g.n, nh = g.nh;
+  const int nf = g.nfreq;
+  const int nfc = g.nfc;
+  const int nsurf = g.nsurf;
   Cpx<T>* W2 = reinterpret_cast<Cpx<T>*>(smem_raw);
   fill_w2(W2, n);
   __syncthreads();
@@ -224,14 +225,12 @@ __global__ void __launch_bounds__(256) k_m2l_inv_warp(M2LGeom g, const T* __rest
       for (int m = lane; m < nsurf; m += 32) {  // c2r along x at the surface points
         int i = g.surf_ijk[3 * m], j = g.surf_ijk[3 * m + 1], k = g.surf_ijk[3 * m + 2];
         const Cpx<T>* a = &A[(k * np + j) * nh];
-        T v = a[0].re + ((i & 1) ? -a[nh - 1].re : a[nh - 1].re);
         T acc = 0;
-#pragma unroll
-        for (int kx = 1; kx < nh - 1; kx++) {
+        for (int kx = 1; kx < nh; kx++) {
           Cpx<T> c = W2[i * n + kx];
           acc = fmt(a[kx].im, c.im, fmt(a[kx].re, c.re, acc));
         }
-        dst[(size_t)m * g.td + t] += v + T(2) * acc;
+        dst[(size_t)m * g.td + t] += a[0].re + T(2) * acc;
       }
       __syncwarp();
     }
@@ -337,12 +336,12 @@ __host__ __device__ constexpr double tw_im(int m, int n) {
   return -s;
 }
 
-// twiddle tables for n = 8, 12, 16, statically initialised from tw_re / tw_im;
+// twiddle tables for n = 7, 11, 15, statically initialised from tw_re / tw_im;
 // indexed with compile-time offsets they are constant-bank operands
 #define KIFMM_TW16(F, n)                                                                                         \
   {F(0, n), F(1, n), F(2, n), F(3, n), F(4, n), F(5, n), F(6, n), F(7, n), F(8, n), F(9, n), F(10, n), F(11, n), \
    F(12, n), F(13, n), F(14, n), F(15, n)}
-#define KIFMM_TWSET(F) {KIFMM_TW16(F, 8), KIFMM_TW16(F, 12), KIFMM_TW16(F, 16)}
+#define KIFMM_TWSET(F) {KIFMM_TW16(F, 7), KIFMM_TW16(F, 11), KIFMM_TW16(F, 15)}
 #define KIFMM_FRE(m, n) (float)tw_re(m, n)
 #define KIFMM_FIM(m, n) (float)tw_im(m, n)
 #define KIFMM_DRE(m, n) tw_re(m, n)
@@ -360,7 +359,7 @@ __constant__ double c_twd_im[3][16] = KIFMM_TWSET(KIFMM_DIM);
 
 template <typename T, int N>
 __device__ __forceinline__ T twr(int m) {
-  constexpr int t = N == 8 ? 0 : N == 12 ? 1 : 2;
+  constexpr int t = N == 7 ? 0 : N == 11 ? 1 : 2;
   if constexpr (sizeof(T) == 4)
     return c_twf_re[t][m % N];
   else
@@ -368,7 +367,7 @@ __device__ __forceinline__ T twr(int m) {
 }
 template <typename T, int N>
 __device__ __forceinline__ T twi(int m) {
-  constexpr int t = N == 8 ? 0 : N == 12 ? 1 : 2;
+  constexpr int t = N == 7 ? 0 : N == 11 ? 1 : 2;
   if constexpr (sizeof(T) == 4)
     return c_twf_im[t][m % N];
   else
@@ -398,7 +397,7 @@ template <typename T, int NP>
 __global__ void __launch_bounds__(256) k_m2l_fwd_rb(M2LGeom g, const T* __restrict__ supeden,
                                                     const int* __restrict__ nodes, int nwork,
                                                     const int* __restrict__ depth, T* __restrict__ spectra) {
-  constexpr int N = 2 * NP, NH = NP + 1, NFC = 4 * NP * NP * NP + 4;
+  constexpr int N = 2 * NP - 1, NH = NP, NFC = ((N * N * N + 1) / 2 + 3) / 4 * 4;
   constexpr int NSURF = NP * NP * NP - (NP - 2) * (NP - 2) * (NP - 2);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpc = blockDim.x >> 5;
@@ -505,7 +504,7 @@ template <typename T, int NP>
 __global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* __restrict__ effval,
                                                     const int* __restrict__ work, int nwork,
                                                     T* __restrict__ tdncval) {
-  constexpr int N = 2 * NP, NH = NP + 1, NFC = 4 * NP * NP * NP + 4;
+  constexpr int N = 2 * NP - 1, NH = NP, NFC = ((N * N * N + 1) / 2 + 3) / 4 * 4;
   constexpr int NSURF = NP * NP * NP - (NP - 2) * (NP - 2) * (NP - 2);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpc = blockDim.x >> 5;
@@ -594,7 +593,7 @@ __global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* __restri
         }
       }
       __syncwarp();
-      // c2r along x, lines (j, k): x_i = Re(a_0) + (-1)^i Re(a_{n/2}) + 2 sum_{0<kx<n/2} Re(a_kx w^(-i kx)),
+      // c2r along x, lines (j, k): x_i = Re(a_0) + 2 sum_{0<kx<nh} Re(a_kx w^(-i kx)),
       // kept at the surface points only
       for (int line = lane; line < NP * NP; line += 32) {
         const int j = line % NP, k = line / NP;
@@ -607,10 +606,9 @@ __global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* __restri
           if (m < 0) continue;
           T acc = 0;
 #pragma unroll
-          for (int kx = 1; kx < NH - 1; kx++)
+          for (int kx = 1; kx < NH; kx++)
             acc = fmt(a[kx].im, twi<T, N>(i * kx), fmt(a[kx].re, twr<T, N>(i * kx), acc));
-          const T v = a[0].re + ((i & 1) ? -a[NH - 1].re : a[NH - 1].re);
-          dst[(size_t)m * g.td + t] += v + T(2) * acc;
+          dst[(size_t)m * g.td + t] += a[0].re + T(2) * acc;
         }
       }
       __syncwarp();
@@ -641,8 +639,8 @@ void launch_m2l_forward(const M2LGeom& g, const T* supeden, const int* nodes, in
     kern<<<gr, 32 * w, sm, st>>>(g, supeden, nodes, nn, depth, spectra);
     return;
   }
-  cudaFuncSetAttribute(k_m2l_fwd_warp<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_m2l_fwd_warp<T, 0><<<grid, 32 * wpc, smem, st>>>(g, supeden, nodes, nn, depth, spectra);
+  cudaFuncSetAttribute(k_m2l_fwd_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_m2l_fwd_warp<T><<<grid, 32 * wpc, smem, st>>>(g, supeden, nodes, nn, depth, spectra);
 }
 
 template <typename T>
@@ -677,8 +675,8 @@ void launch_m2l_inverse(const M2LGeom& g, const T* effval, const int* work, int 
     kern<<<gr, 32 * w, sm, st>>>(g, effval, work, nwork, tdncval);
     return;
   }
-  cudaFuncSetAttribute(k_m2l_inv_warp<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_m2l_inv_warp<T, 0><<<grid, 32 * wpc, smem, st>>>(g, effval, work, nwork, tdncval);
+  cudaFuncSetAttribute(k_m2l_inv_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_m2l_inv_warp<T><<<grid, 32 * wpc, smem, st>>>(g, effval, work, nwork, tdncval);
 }
 
 // ---------------------------------------------------------------------------
@@ -1172,7 +1170,7 @@ void sweep_dofs(int sd, int td, const T* ktiles, const T* spectra, int nq, const
 }  // namespace
 
 bool m2l_sweep_supported(int nf, int sd, int td) {
-  return (nf == 260 || nf == 868 || nf == 2052) &&
+  return (nf == 172 || nf == 668 || nf == 1688) &&
          ((sd == 1 && td == 1) || (sd == 4 && td == 3) || (sd == 3 && td == 3));
 }
 
@@ -1181,24 +1179,24 @@ void launch_m2l_hadamard_sweep(int nf, int sd, int td, const T* ktiles, const T*
                                const int* coll, const unsigned char* mask, T* effval, int zero_node, int* status,
                                int num_sms, cudaStream_t st) {
   if (nq <= 0) return;
-  if (nf == 868)
-    sweep_dofs<T, 868>(sd, td, ktiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
-  else if (nf == 260)
-    sweep_dofs<T, 260>(sd, td, ktiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
-  else if (nf == 2052)
-    sweep_dofs<T, 2052>(sd, td, ktiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+  if (nf == 668)
+    sweep_dofs<T, 668>(sd, td, ktiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+  else if (nf == 172)
+    sweep_dofs<T, 172>(sd, td, ktiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+  else if (nf == 1688)
+    sweep_dofs<T, 1688>(sd, td, ktiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
 }
 
 void launch_m2l_hadamard_tz(int nf, int sd, int td, const float* ttiles, const float* spectra, int nq, const int* qchd,
                             const int* coll, const unsigned char* mask, float* effval, int zero_node, int* status,
                             int num_sms, cudaStream_t st) {
   if (nq <= 0) return;
-  if (nf == 868)
-    tz_dofs<float, 868>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
-  else if (nf == 260)
-    tz_dofs<float, 260>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
-  else if (nf == 2052)
-    tz_dofs<float, 2052>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+  if (nf == 668)
+    tz_dofs<float, 668>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+  else if (nf == 172)
+    tz_dofs<float, 172>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+  else if (nf == 1688)
+    tz_dofs<float, 1688>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
 }
 
 #define KIFMM_INST(T)                                                                                             \

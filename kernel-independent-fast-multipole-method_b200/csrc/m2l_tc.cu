@@ -503,7 +503,7 @@ inline float tf32_round_host(float x) {
 }  // namespace
 
 bool m2l_tc_supported(int nf, int sd, int td) {
-  return sd == 1 && td == 1 && (nf == 260 || nf == 868 || nf == 2052);
+  return sd == 1 && td == 1 && (nf == 172 || nf == 668 || nf == 1688);
 }
 
 void m2l_tc_images(int nf, const std::complex<double>* m2l, std::vector<float>* img) {
@@ -542,12 +542,12 @@ void m2l_tc_images(int nf, const std::complex<double>* m2l, std::vector<float>* 
 void launch_m2l_hadamard_tc(int nf, const float* img, const float* spectra, int nq, const int* qchd,
                             const int* coll, const unsigned char* mask, const unsigned* tile_dirs, float* effval,
                             int zero_node, int* status, int num_sms, cudaStream_t st) {
-  if (nf == 868)
-    had_tc_launch<868>(img, spectra, nq, qchd, coll, mask, tile_dirs, effval, zero_node, status, num_sms, st);
-  else if (nf == 260)
-    had_tc_launch<260>(img, spectra, nq, qchd, coll, mask, tile_dirs, effval, zero_node, status, num_sms, st);
-  else if (nf == 2052)
-    had_tc_launch<2052>(img, spectra, nq, qchd, coll, mask, tile_dirs, effval, zero_node, status, num_sms,
+  if (nf == 668)
+    had_tc_launch<668>(img, spectra, nq, qchd, coll, mask, tile_dirs, effval, zero_node, status, num_sms, st);
+  else if (nf == 172)
+    had_tc_launch<172>(img, spectra, nq, qchd, coll, mask, tile_dirs, effval, zero_node, status, num_sms, st);
+  else if (nf == 1688)
+    had_tc_launch<1688>(img, spectra, nq, qchd, coll, mask, tile_dirs, effval, zero_node, status, num_sms,
                         st);
 }
 

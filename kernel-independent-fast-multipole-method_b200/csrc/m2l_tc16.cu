@@ -692,7 +692,7 @@ void had_tc16_dofs(int groups, int sd, int td, const unsigned char* img, const u
 
 bool m2l_tc16_supported(int nf, int sd, int td) {
   const bool dofs = (sd == 1 && td == 1) || (sd == 4 && td == 3) || (sd == 3 && td == 3);
-  return dofs && (nf == 260 || nf == 868 || nf == 2052);
+  return dofs && (nf == 172 || nf == 668 || nf == 1688);
 }
 
 void m2l_tc16_images(int nf, int sd, int td, const std::complex<double>* m2l, std::vector<unsigned short>* img,
@@ -768,14 +768,14 @@ void launch_m2l_hadamard_tc16(int groups, int nf, int sd, int td, const unsigned
                               const unsigned* tile_dirs, float* effval, size_t plane, const unsigned* bound,
                               const float* inv_sb, int wait_limit, int* status, int num_sms, cudaStream_t st) {
   const unsigned char* im = reinterpret_cast<const unsigned char*>(img);
-  if (nf == 868)
-    had_tc16_dofs<868>(groups, sd, td, im, spectra, nq, qchd, ctab, tile_dirs, effval, plane, bound, inv_sb,
+  if (nf == 668)
+    had_tc16_dofs<668>(groups, sd, td, im, spectra, nq, qchd, ctab, tile_dirs, effval, plane, bound, inv_sb,
                        wait_limit, status, num_sms, st);
-  else if (nf == 260)
-    had_tc16_dofs<260>(groups, sd, td, im, spectra, nq, qchd, ctab, tile_dirs, effval, plane, bound, inv_sb,
+  else if (nf == 172)
+    had_tc16_dofs<172>(groups, sd, td, im, spectra, nq, qchd, ctab, tile_dirs, effval, plane, bound, inv_sb,
                        wait_limit, status, num_sms, st);
-  else if (nf == 2052)
-    had_tc16_dofs<2052>(groups, sd, td, im, spectra, nq, qchd, ctab, tile_dirs, effval, plane, bound, inv_sb,
+  else if (nf == 1688)
+    had_tc16_dofs<1688>(groups, sd, td, im, spectra, nq, qchd, ctab, tile_dirs, effval, plane, bound, inv_sb,
                         wait_limit, status, num_sms, st);
 }
 

@@ -374,8 +374,10 @@ std::shared_ptr<Operators> build_operators(const KernelDesc& mm, int np, int nth
   surface_grid(np, 1.0, &o.dc, nullptr);
   o.nsurf = (int)o.ue.size() / 3;
   o.nuc = (int)o.uc.size() / 3;
-  o.n = 2 * np;
-  o.nh = np + 1;
+  // the smallest cyclic grid without wrap-around: np source and np target points
+  // per axis have 2 np - 1 lags (the reference transforms 2 np, fmm3d/matmgnt3d.cpp:307-325)
+  o.n = 2 * np - 1;
+  o.nh = np;
   o.nfreq = o.n * o.n * o.nh;
   const int sd = mm.sd, td = mm.td, ns = o.nsurf, nc = o.nuc;
   const double cut = std::pow(0.1, np + 1);  // MatMgnt3d::alt, fmm3d/matmgnt3d.cpp:38-41
@@ -452,8 +454,9 @@ std::shared_ptr<Operators> build_operators(const KernelDesc& mm, int np, int nth
   const int n = o.n, nh = o.nh;
   const double step = 2.0 / (np - 1);
   // Hermitian compaction: a real grid's half spectrum (kx < nh) repeats its
-  // kx = 0 and kx = n/2 planes as X(kx,-ky,-kz) = conj X(kx,ky,kz); only the
-  // canonical member of each pair, (kz,ky) <= (-kz,-ky) mod n, is kept.
+  // kx = 0 plane as X(0,-ky,-kz) = conj X(0,ky,kz); only the canonical member
+  // of each pair, (kz,ky) <= (-kz,-ky) mod n, is kept: (n^3 + 1) / 2 values,
+  // padded to a multiple of 4 with frequencies whose operator is zero.
   o.ff2c.assign(o.nfreq, 0);
   o.fc2f.clear();
   for (int kz = 0; kz < n; kz++)
@@ -461,20 +464,20 @@ std::shared_ptr<Operators> build_operators(const KernelDesc& mm, int np, int nth
       for (int kx = 0; kx < nh; kx++) {
         const int f = (kz * n + ky) * nh + kx;
         const int mz = (n - kz) % n, my = (n - ky) % n;
-        const bool edge = kx == 0 || 2 * kx == n;
-        if (!edge || kz < mz || (kz == mz && ky <= my)) {
+        if (kx != 0 || kz < mz || (kz == mz && ky <= my)) {
           o.ff2c[f] = (int)o.fc2f.size();
           o.fc2f.push_back(f);
         }
       }
+  const int nfu = (int)o.fc2f.size();  // without the padding
+  while (o.fc2f.size() % 4) o.fc2f.push_back(0);
   o.nfc = (int)o.fc2f.size();
   for (int kz = 0; kz < n; kz++)
-    for (int ky = 0; ky < n; ky++)
-      for (int kx : {0, n / 2}) {
-        const int f = (kz * n + ky) * nh + kx;
-        const int mz = (n - kz) % n, my = (n - ky) % n;
-        if (!(kz < mz || (kz == mz && ky <= my))) o.ff2c[f] = -o.ff2c[(mz * n + my) * nh + kx] - 1;
-      }
+    for (int ky = 0; ky < n; ky++) {
+      const int f = (kz * n + ky) * nh;
+      const int mz = (n - kz) % n, my = (n - ky) % n;
+      if (!(kz < mz || (kz == mz && ky <= my))) o.ff2c[f] = -o.ff2c[(mz * n + my) * nh] - 1;
+    }
   const int nfc = o.nfc;
   o.m2l.assign((size_t)343 * td * sd * nfc, std::complex<double>(0.0, 0.0));
   std::vector<std::complex<double>> w(n);
@@ -520,7 +523,7 @@ std::shared_ptr<Operators> build_operators(const KernelDesc& mm, int np, int nth
           }
       // z pass at the canonical frequencies, f = (kz*n + ky)*nh + kx
       std::complex<double>* dst = &o.m2l[((size_t)oidx * td * sd + e) * nfc];
-      for (int c = 0; c < nfc; c++) {
+      for (int c = 0; c < nfu; c++) {
         const int f = o.fc2f[c], kx = f % nh, ky = (f / nh) % n, kz = f / (nh * n);
         std::complex<double> s(0, 0);
         for (int gz = 0; gz < n; gz++) s += B[((size_t)gz * n + ky) * nh + kx] * w[(gz * kz) % n];

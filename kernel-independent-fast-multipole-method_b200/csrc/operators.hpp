@@ -54,9 +54,9 @@ struct Operators {
   int np = 0;
   int nsurf = 0;          // |UE| = |DE| = |DC| = np^3 - (np-2)^3
   int nuc = 0;            // |UC| = (np+2)^3 - np^3
-  int n = 0, nh = 0;      // FFT grid 2np, halved axis n/2+1
+  int n = 0, nh = 0;      // transform grid 2 np - 1, halved axis np
   int nfreq = 0;          // n*n*nh
-  int nfc = 0;            // independent (Hermitian-canonical) frequencies, 4 np^3 + 4
+  int nfc = 0;            // independent (Hermitian-canonical) frequencies, (n^3 + 1) / 2 up to a multiple of 4
   std::vector<int> fc2f;  // compact -> full frequency index
   std::vector<int> ff2c;  // full -> compact index c, or -c-1 where the value is conj(compact c)
   std::vector<int> deg;   // per sd
