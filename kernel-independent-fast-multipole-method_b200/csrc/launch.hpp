@@ -217,9 +217,9 @@ void launch_m2l_hadamard_tz(int nf, int sd, int td, const float* ttiles, const f
 // the device from the operator spectra khat [343][td][sd][nf].  Parents in groups
 // of 16 rows, a step per direction that one of them has: head [group] {first
 // step, number of steps}, tab [step][16] the colleague's sibling group (the
-// all-zero group for an absent one or a padding row), desc [step] the operator
-// fragment and which 8 rows have the direction, out [group][16] the target
-// sibling group (-1: padding).
+// all-zero group for an absent one or a padding row), desc [step] the
+// direction's operator fragments, out [group][16] the target sibling group (-1:
+// padding).
 struct Had64Groups {
   const int *head = nullptr, *tab = nullptr, *desc = nullptr, *out = nullptr;
 };

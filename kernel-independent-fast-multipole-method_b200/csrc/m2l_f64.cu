@@ -17,7 +17,7 @@
 // multiply-adds, and the load path fills 128 bytes a clock per SM even when
 // all lanes read one address: the same sums with the factorisation along all
 // three axes (27 products instead of 64, 146 FP64 instructions) ran at 34 % of
-// the pipe, 80 % of the load path, 23.0 ms at 4M points.  Here a fill serves 8
+// the pipe, 80 % of the load path, 23.0 ms where this form takes 13.9.  Here a fill serves 8
 // parents and the pipe is the bound.
 //
 // A CTA keeps NF frequencies and one target dof, whose operator for all source
@@ -27,17 +27,19 @@
 // from global memory (spectra_f64_index); neighbouring parents share
 // colleagues, which L1 serves.  The layout keeps frequency pairs innermost: with
 // the 8 children of one frequency contiguous, one load a row, this kernel is no
-// faster (13.9 ms at 4M either way) and the forward pass, whose nodes then
-// write half sectors, takes 8.2 ms instead of 2.6.
-// A tile skips the directions that none of its 8 parents has: what is left is
-// 1.05x the work in a volume and 1.3-1.8x on a surface (had64_groups groups the
-// parents by direction sets).
+// faster and the forward pass, whose nodes then write half sectors, takes 8.2 ms
+// instead of 2.6 (4M points).
+// A group takes every direction that one of its 16 parents has, 1.05x the work in
+// a volume and 1.4-2x on a surface (had64_groups groups the parents by direction
+// sets; letting each tile of 8 skip its own, 1.3-1.8x the work, is slower: one
+// tile alone waits for its operator fragments and rows).
 //
 // Measured, against one launch of the direct parent-pair sweep (m2l.cu) per dof
-// pair: Laplace np = 6, 4,194,304 points in a volume 22.5 -> 13.9 ms (matrix
-// pipe 75 % busy); Stokes np = 6, 262,144 points on an ellipsoid 28.4 -> 4.8 ms;
-// Navier np = 8, 1,048,576 points on a sphere 45.9 -> 20.6 ms; Laplace np = 4,
-// 32,768 points on a sphere 0.64 -> 0.03 ms.
+// pair on the transforms of 2 np points that it then had: Laplace np = 6, 4,194,304
+// points in a volume 22.5 -> 10.4 ms (13.9 on 2 np points; matrix pipe 75 % busy);
+// Stokes np = 6, 262,144 points on an ellipsoid 28.4 -> 3.0 ms; Navier np = 8, 1,048,576
+// points on a sphere 45.9 -> 14.5 ms; Laplace np = 4, 32,768 points on a sphere 0.64 ->
+// 0.03 ms.
 #include <algorithm>
 #include <cmath>
 
@@ -67,10 +69,6 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     k_m2l_had64(const double2* __restrict__ tables, const double2* __restrict__ spectra, size_t plane, int nfc, int ngroup,
                 int per_slice, const int2* __restrict__ ghead, const int* __restrict__ gtab,
                 const int* __restrict__ gdesc, const int* __restrict__ gout, double2* __restrict__ effval) {
-  // several dofs: a tile skips the directions that none of its rows has; one
-  // dof: both tiles take every direction of the group (the branches cost more
-  // than the 3 % of the multiplications they save in a volume)
-  constexpr bool SKIP = SD > 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* Bs = reinterpret_cast<double2*>(smem_raw);  // [NF][SD][26][3][32]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, c = lane & 3;
@@ -103,10 +101,10 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     // multiplied, from a descriptor and colleague indices that were loaded one
     // step earlier still (past the last step they wrap to the first again)
     TileX xa[H_TILES], xb[H_TILES];
-    int ea, eb;  // B fragment offset * 4 + the tiles that take the step
+    int ea, eb;  // B fragment offset
     int i = 0, s = 0, idx[H_TILES], de;
     auto fetch = [&] {
-      de = __ldg(desc + i) + s * (26 * 96 * 4);
+      de = __ldg(desc + i) + s * (26 * 96);
 #pragma unroll
       for (int n = 0; n < H_TILES; n++) idx[n] = __ldg(tab + i * H_GROUP + 8 * n);
     };
@@ -114,12 +112,11 @@ __global__ void __launch_bounds__(H_THREADS, 1)
       e = de;
       const double2* X = spectra + (size_t)s * plane + lbase;
 #pragma unroll
-      for (int n = 0; n < H_TILES; n++)
-        if (!SKIP || ((e >> n) & 1)) {
-          const double2* p = X + (size_t)idx[n] * gstride;
-          x[n].x0 = __ldg(p);
-          x[n].x1 = __ldg(p + 8);
-        }
+      for (int n = 0; n < H_TILES; n++) {
+        const double2* p = X + (size_t)idx[n] * gstride;
+        x[n].x0 = __ldg(p);
+        x[n].x1 = __ldg(p + 8);
+      }
       if (++i == head.y) {
         i = 0;
         if (++s == SD) s = 0;
@@ -127,33 +124,19 @@ __global__ void __launch_bounds__(H_THREADS, 1)
       fetch();
     };
     auto multiply = [&](const TileX* x, int e) {
-      const double2* B = Bw + (e >> 2);
+      const double2* B = Bw + e;
       const double2 b0 = B[0], b1 = B[32], b2 = B[64];
-      if constexpr (SKIP) {
 #pragma unroll
-        for (int n = 0; n < H_TILES; n++)
-          if ((e >> n) & 1) {
-            const double2 x0 = x[n].x0, x1 = x[n].x1;
-            mma(acc[n][1], x1.x, b1.x);
-            mma(acc[n][2], x0.x, b2.x);
-            mma(acc[n][0], x0.x + x1.x, b0.x);
-            mma(acc[n][1], x1.y, b1.y);
-            mma(acc[n][2], x0.y, b2.y);
-            mma(acc[n][0], x0.y + x1.y, b0.y);
-          }
-      } else {
+      for (int n = 0; n < H_TILES; n++) {
+        mma(acc[n][1], x[n].x1.x, b1.x);
+        mma(acc[n][2], x[n].x0.x, b2.x);
+        mma(acc[n][0], x[n].x0.x + x[n].x1.x, b0.x);
+      }
 #pragma unroll
-        for (int n = 0; n < H_TILES; n++) {
-          mma(acc[n][1], x[n].x1.x, b1.x);
-          mma(acc[n][2], x[n].x0.x, b2.x);
-          mma(acc[n][0], x[n].x0.x + x[n].x1.x, b0.x);
-        }
-#pragma unroll
-        for (int n = 0; n < H_TILES; n++) {
-          mma(acc[n][1], x[n].x1.y, b1.y);
-          mma(acc[n][2], x[n].x0.y, b2.y);
-          mma(acc[n][0], x[n].x0.y + x[n].x1.y, b0.y);
-        }
+      for (int n = 0; n < H_TILES; n++) {
+        mma(acc[n][1], x[n].x1.y, b1.y);
+        mma(acc[n][2], x[n].x0.y, b2.y);
+        mma(acc[n][0], x[n].x0.y + x[n].x1.y, b0.y);
       }
     };
     fetch();
@@ -236,14 +219,14 @@ void launch_had64_tables(const double* khat, int nf, int sd, int td, double* tab
                                                reinterpret_cast<double2*>(tables));
 }
 
-// Row tiles of 8 target parents, two to a group.  A group takes every
-// direction that one of its parents has, so inside windows of 1024 parents
-// (Morton order, whose colleagues stay near) tiles are filled greedily: a
-// parent and, seven times, the one that adds the fewest directions (of those,
-// the one that shares the most).  On a sphere of 1,048,576 points a tile then
-// takes 1.34 directions per direction of a parent, in Morton order 1.84.
+// Groups of 16 target parents, two row tiles of 8.  A group takes every
+// direction that one of its parents has, so inside windows of 4096 parents
+// (Morton order, whose colleagues stay near) groups are filled greedily: a
+// parent and, fifteen times, the one that adds the fewest directions (of those,
+// the one that shares the most).  On a sphere of 1,048,576 points a group then
+// takes 1.45 directions per direction of a parent, in Morton order 2.03.
 void had64_groups(int nq, int zero_node, const int* qchd, const int* coll, Had64HostGroups* o) {
-  constexpr int WINDOW = 1024;
+  constexpr int WINDOW = 4096;
   std::vector<unsigned> dirs(nq, 0u);
   std::vector<int> order(nq);
   auto window = [&](int b) {
@@ -255,11 +238,11 @@ void had64_groups(int nq, int zero_node, const int* qchd, const int* coll, Had64
         if (coll[(size_t)w * 26 + d] != zero_node) dirs[w] |= 1u << d;
     }
     while (!left.empty()) {
-      // a tile begins with the next parent of the Morton order
+      // a group begins with the next parent of the Morton order
       unsigned m = dirs[left[0]];
       order[n++] = left[0];
       left.erase(left.begin());
-      for (int k = 1; k < 8 && !left.empty(); k++) {
+      for (int k = 1; k < H_GROUP && !left.empty(); k++) {
         int best = 0, cost = 1 << 30;
         for (int e = 0; e < (int)left.size() && cost > -__builtin_popcount(m); e++) {
           const unsigned v = dirs[left[e]];
@@ -285,17 +268,17 @@ void had64_groups(int nq, int zero_node, const int* qchd, const int* coll, Had64
   o->desc.clear();
   o->out.assign((size_t)ng * H_GROUP, -1);
   for (int g = 0; g < ng; g++) {
-    unsigned m[H_TILES] = {0u, 0u};
+    unsigned m = 0;
     for (int r = 0; r < H_GROUP && g * H_GROUP + r < nq; r++) {
       const int w = order[g * H_GROUP + r];
-      m[r / 8] |= dirs[w];
+      m |= dirs[w];
       o->out[g * H_GROUP + r] = (qchd[w] + 7) >> 3;
     }
     o->head.push_back((int)o->desc.size());
     int n = 0;
     for (int d = 0; d < 26; d++) {
-      if (!(((m[0] | m[1]) >> d) & 1)) continue;
-      o->desc.push_back(d * 96 * 4 + (int)((m[0] >> d) & 1) + 2 * (int)((m[1] >> d) & 1));
+      if (!((m >> d) & 1)) continue;
+      o->desc.push_back(d * 96);
       for (int r = 0; r < H_GROUP; r++) {
         const int e = g * H_GROUP + r;
         o->tab.push_back(e < nq ? (coll[(size_t)order[e] * 26 + d] + 7) >> 3 : zero);
