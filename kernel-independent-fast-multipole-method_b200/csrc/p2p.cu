@@ -7,8 +7,8 @@
 //                       downward equivalent surface (DE2TC_dgemv, :84-112), fused into one pass that
 //                       writes each target once.
 //
-// S2M and the leaf pass run one warp per leaf (see below); S2L, rare, one CTA
-// per node with shared-memory tiles.  Every target accumulates in registers.
+// S2M and the leaf pass run warps on leaves (see below); S2L, rare, CTAs on a
+// node's check points with shared-memory tiles.  Every target accumulates in registers.
 // Positions are stored relative to the centre of their leaf and re-centred on
 // the target node's centre while staging, so FP32 differences lose no more
 // than the node size's precision.
@@ -42,48 +42,11 @@ struct P4 {
   T x, y, z, w;
 };
 
-__device__ __forceinline__ int group_size(int nt) {
-  int g = ((nt + 31) / 32) * 32;
-  return g > P2P_THREADS ? P2P_THREADS : (g < 32 ? 32 : g);
-}
-
-// Stages points [b, b+cnt) of a source leaf (local coords + shift) into the tile.
-template <typename T, int SD, bool DL>
-__device__ __forceinline__ void stage_points(Tile<T, 4>& t, const P2PArgs<T>& a, int b, int cnt, T shx, T shy,
-                                             T shz, int rhs) {
-  for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-    int p = b + j;
-    t.x[j] = a.sx[p] + shx;
-    t.y[j] = a.sy[p] + shy;
-    t.z[j] = a.sz[p] + shz;
-    if constexpr (DL) {
-      t.nx[j] = a.snx[p];
-      t.ny[j] = a.sny[p];
-      t.nz[j] = a.snz[p];
-    }
-#pragma unroll
-    for (int s = 0; s < SD; s++) t.f[j * SD + s] = a.sden[(size_t)rhs * a.ns * SD + (size_t)p * SD + s];
-  }
-}
-
-// Stages `cnt` points of a surface grid (unit * rad + shift) with densities den[k*SD + s].
-template <typename T, int SD>
-__device__ __forceinline__ void stage_surface(Tile<T, 4>& t, const T* unit, int k0, int cnt, T rad, T shx, T shy,
-                                              T shz, const T* den) {
-  for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-    int k = k0 + j;
-    t.x[j] = unit[3 * k] * rad + shx;
-    t.y[j] = unit[3 * k + 1] * rad + shy;
-    t.z[j] = unit[3 * k + 2] * rad + shz;
-#pragma unroll
-    for (int s = 0; s < SD; s++) t.f[j * SD + s] = den[(size_t)k * SD + s];
-  }
-}
-
 template <typename T, int KT>
 __device__ __forceinline__ void accumulate_tile(const Tile<T, 4>& t, int cnt, int j0, int jstep, T px, T py, T pz,
                                                 T* acc, const KConst<T>& kc) {
   constexpr int SD = KTraits<KT>::SD;
+#pragma unroll 4
   for (int j = j0; j < cnt; j += jstep) {
     T nrm[3];
     if constexpr (KTraits<KT>::DL) {
@@ -119,45 +82,87 @@ __device__ __forceinline__ void reduce_and_store(Red<T, 4>& red, const T* acc, i
 }
 
 // ---------------------------------------------------------------------------
+// S2L: CTA (w, b) sums the X-list sources of work item w at downward check
+// points 32 b .. 32 b + 31, each point's sources over its four warps.  The list's
+// leaves are small and many (they are finer than the node), so 128 of them at a
+// time get a prefix sum and the sources are staged 256 at a time across leaf
+// borders.  One CTA per node and a barrier pair per leaf, the form before, was
+// latency: 44 us for 70 nodes of a 262,144-point tree, now 12.
 template <typename T, int KT>
 __global__ void __launch_bounds__(P2P_THREADS) k_s2l(P2PArgs<T> a, const int* work, const int64_t* ptr,
-                                                      const int* idx, int nwork, int rhs) {
+                                                      const int* idx, int rhs) {
   constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD;
   constexpr bool DL = KTraits<KT>::DL;
+  constexpr int G = 32, NSPLIT = P2P_THREADS / G;
   __shared__ Tile<T, 4> tile;
   __shared__ Red<T, 4> red;
-  int w = blockIdx.x;
-  int g = work[w];
-  T rad = (T)a.radius[g];
-  double cx = a.center[3 * g], cy = a.center[3 * g + 1], cz = a.center[3 * g + 2];
-  int nt = a.nsurf;
-  int G = group_size(nt), nsplit = P2P_THREADS / G;
-  int slot = threadIdx.x % G, sg = threadIdx.x / G;
-  T* outbase = a.tdncval + (size_t)g * a.nsurf * TD;
-  for (int tb = 0; tb < nt; tb += G) {
-    int ti = tb + slot;
-    bool valid = ti < nt && sg < nsplit;
-    T px = 0, py = 0, pz = 0;
-    if (valid) {
-      px = a.dc_unit[3 * ti] * rad;
-      py = a.dc_unit[3 * ti + 1] * rad;
-      pz = a.dc_unit[3 * ti + 2] * rad;
-    }
-    T acc[4] = {0, 0, 0, 0};
-    for (int64_t e = ptr[w]; e < ptr[w + 1]; e++) {
-      int s = idx[e];
-      T shx = (T)(a.center[3 * s] - cx), shy = (T)(a.center[3 * s + 1] - cy), shz = (T)(a.center[3 * s + 2] - cz);
-      int sb = a.sbeg[s], sc = a.scnt[s];
-      for (int c0 = 0; c0 < sc; c0 += TILE) {
-        int cnt = min(TILE, sc - c0);
-        __syncthreads();
-        stage_points<T, SD, DL>(tile, a, sb + c0, cnt, shx, shy, shz, rhs);
-        __syncthreads();
-        if (valid) accumulate_tile<T, KT>(tile, cnt, sg, nsplit, px, py, pz, acc, a.ku);
-      }
-    }
-    reduce_and_store<T, TD>(red, acc, G, nsplit, ti < nt, outbase + (size_t)ti * TD, true);
+  __shared__ int lbeg[P2P_THREADS], pre[P2P_THREADS + 1], wsum[NSPLIT];
+  __shared__ T lx[P2P_THREADS], ly[P2P_THREADS], lz[P2P_THREADS];
+  const int w = blockIdx.x, g = work[w], tid = threadIdx.x, lane = tid & 31;
+  const T rad = (T)a.radius[g];
+  const double cx = a.center[3 * g], cy = a.center[3 * g + 1], cz = a.center[3 * g + 2];
+  const int ti = blockIdx.y * G + lane, sg = tid >> 5;
+  const bool valid = ti < a.nsurf;
+  T px = 0, py = 0, pz = 0;
+  if (valid) {
+    px = a.dc_unit[3 * ti] * rad;
+    py = a.dc_unit[3 * ti + 1] * rad;
+    pz = a.dc_unit[3 * ti + 2] * rad;
   }
+  const T* den = a.sden + (size_t)rhs * a.ns * SD;
+  T acc[4] = {0, 0, 0, 0};
+  for (int64_t e0 = ptr[w]; e0 < ptr[w + 1]; e0 += P2P_THREADS) {
+    const int nleaf = (int)min((int64_t)P2P_THREADS, ptr[w + 1] - e0);
+    int c = 0;
+    if (tid < nleaf) {
+      const int s = idx[e0 + tid];
+      lbeg[tid] = a.sbeg[s];
+      c = a.scnt[s];
+      lx[tid] = (T)(a.center[3 * s] - cx);
+      ly[tid] = (T)(a.center[3 * s + 1] - cy);
+      lz[tid] = (T)(a.center[3 * s + 2] - cz);
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, c, o);
+      if (lane >= o) c += v;
+    }
+    if (lane == 31) wsum[sg] = c;
+    __syncthreads();
+    for (int q = 0; q < sg; q++) c += wsum[q];
+    pre[tid + 1] = c;
+    if (tid == 0) pre[0] = 0;
+    __syncthreads();
+    const int total = pre[P2P_THREADS];
+    for (int k0 = 0; k0 < total; k0 += TILE) {
+      const int cnt = min(TILE, total - k0);
+      for (int j = tid; j < cnt; j += P2P_THREADS) {
+        int lo = 0, hi = nleaf;  // pre[lo] <= k0 + j < pre[hi]
+        while (hi - lo > 1) {
+          const int mid = (lo + hi) >> 1;
+          if (pre[mid] <= k0 + j)
+            lo = mid;
+          else
+            hi = mid;
+        }
+        const int p = lbeg[lo] + (k0 + j - pre[lo]);
+        tile.x[j] = a.sx[p] + lx[lo];
+        tile.y[j] = a.sy[p] + ly[lo];
+        tile.z[j] = a.sz[p] + lz[lo];
+        if constexpr (DL) {
+          tile.nx[j] = a.snx[p];
+          tile.ny[j] = a.sny[p];
+          tile.nz[j] = a.snz[p];
+        }
+#pragma unroll
+        for (int s = 0; s < SD; s++) tile.f[j * SD + s] = den[(size_t)p * SD + s];
+      }
+      __syncthreads();
+      if (valid) accumulate_tile<T, KT>(tile, cnt, sg, NSPLIT, px, py, pz, acc, a.ku);
+      __syncthreads();
+    }
+  }
+  reduce_and_store<T, TD>(red, acc, G, NSPLIT, valid, a.tdncval + ((size_t)g * a.nsurf + ti) * TD, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -738,7 +743,8 @@ void launch_p2p_kt(const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cu
       }
       break;
     case P2P_S2L:
-      if (w.n) k_s2l<T, KT><<<w.n, P2P_THREADS, 0, st>>>(a, w.work, w.ptr, w.idx, w.n, rhs);
+      if (w.n)
+        k_s2l<T, KT><<<dim3(w.n, (a.nsurf + 31) / 32), P2P_THREADS, 0, st>>>(a, w.work, w.ptr, w.idx, rhs);
       break;
     case P2P_LEAF:
       if (w.n) {
