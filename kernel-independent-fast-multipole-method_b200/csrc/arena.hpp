@@ -15,8 +15,13 @@ class DeviceArena {
   DeviceArena() = default;
   DeviceArena(const DeviceArena&) = delete;
   DeviceArena& operator=(const DeviceArena&) = delete;
-  ~DeviceArena() {
+  ~DeviceArena() { clear(); }
+  // frees everything (each free waits for the device)
+  void clear() {
     for (void* p : blocks_) cudaFree(p);
+    blocks_.clear();
+    cur_ = nullptr;
+    left_ = 0;
   }
   // `bytes` (at least one) of device memory at a 256-byte boundary
   cudaError_t get(size_t bytes, void** out) {

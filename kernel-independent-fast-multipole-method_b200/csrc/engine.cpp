@@ -129,6 +129,69 @@ std::shared_ptr<Had64Tables> had64_tables(const std::shared_ptr<const Operators>
   return p;
 }
 
+// Mapped host words that the kernels set on a wait's time-out, one per engine.
+// Pinning memory costs 3 ms, so the words come from one pinned page per process
+// (1,024 engines; more pin their own word) and go back to it; the page is
+// checked against the current context on every request, since a
+// cudaDeviceReset unregisters it.
+class StatusWords {
+ public:
+  struct Word {
+    int *host = nullptr, *dev = nullptr;
+    int slot = -1;      // -1: its own allocation
+    unsigned page = 0;  // the page it came from
+  };
+  static StatusWords& get() {
+    static StatusWords* w = new StatusWords;  // never destroyed: engines may outlive static objects
+    return *w;
+  }
+  Word acquire() {
+    std::lock_guard<std::mutex> lk(mu_);
+    void* d = nullptr;
+    if (page_ && cudaHostGetDevicePointer(&d, page_, 0) != cudaSuccess) {
+      cudaGetLastError();
+      page_ = nullptr;
+    }
+    if (!page_) {
+      KCHECK(cudaHostAlloc((void**)&page_, kSlots * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+      used_.assign(kSlots, 0);
+      gen_++;
+      KCHECK(cudaHostGetDevicePointer(&d, page_, 0));
+    }
+    Word w;
+    for (int i = 0; i < kSlots; i++)
+      if (!used_[i]) {
+        used_[i] = 1;
+        w.host = page_ + i;
+        w.dev = (int*)d + i;
+        w.slot = i;
+        w.page = gen_;
+        *w.host = 0;
+        return w;
+      }
+    KCHECK(cudaHostAlloc((void**)&w.host, sizeof(int), cudaHostAllocMapped));
+    *w.host = 0;
+    KCHECK(cudaHostGetDevicePointer((void**)&w.dev, w.host, 0));
+    return w;
+  }
+  void release(const Word& w) {
+    if (!w.host) return;
+    if (w.slot < 0) {
+      cudaFreeHost(w.host);
+      return;
+    }
+    std::lock_guard<std::mutex> lk(mu_);
+    if (w.page == gen_ && page_) used_[w.slot] = 0;
+  }
+
+ private:
+  static constexpr int kSlots = 1024;
+  std::mutex mu_;
+  int* page_ = nullptr;
+  std::vector<char> used_;
+  unsigned gen_ = 0;
+};
+
 }  // namespace
 
 template <typename T>
@@ -237,6 +300,7 @@ struct Impl : ImplBase {
   unsigned* htc_dirs = nullptr;     // tensor-core Hadamard: directions present per tile of 128 parents
   int* h_status = nullptr;  // mapped host word: device-side wait time-outs (bit 0 sweeps, bit 1 GEMM, bits 2 and 3 the tensor-core Hadamard)
   int* d_status = nullptr;
+  StatusWords::Word status_word;
   List s2m, s2l, leaf, m2l, fwd;
   std::vector<List> up_non, dn_par;
   List up_all, dn_all;
@@ -249,7 +313,8 @@ struct Impl : ImplBase {
 
   Impl(Engine& e) : E(e), tr(e.tree), op(*e.ops) {}
   ~Impl() override {
-    if (h_status) cudaFreeHost(h_status);
+    arena.clear();  // waits for the device: no kernel of this engine sets the word after this
+    StatusWords::get().release(status_word);
     if (have_events)
       for (auto& x : ev) cudaEventDestroy(x);
   }
@@ -371,9 +436,9 @@ struct Impl : ImplBase {
       }
       khat = upload(kh);
     }
-    KCHECK(cudaHostAlloc((void**)&h_status, sizeof(int), cudaHostAllocMapped));
-    *h_status = 0;
-    KCHECK(cudaHostGetDevicePointer((void**)&d_status, h_status, 0));
+    status_word = StatusWords::get().acquire();
+    h_status = status_word.host;
+    d_status = status_word.dev;
     double kc[3];
     kernel_constants(E.user.kt, E.user.coefs, kc);
     args.ku = KConst<T>{(T)kc[0], (T)kc[1], (T)kc[2]};
