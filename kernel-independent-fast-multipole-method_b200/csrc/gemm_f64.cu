@@ -86,6 +86,8 @@ __global__ void __launch_bounds__(G_THREADS, 2)
     for (int j = 0; j < NT; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
   const int wn = (warp & 1) * 32, wm = (warp >> 1) * (8 * NT);  // the warp's first node and operator row
   const int steps = ke > kb ? (ke - kb + G_BK - 1) / G_BK : 0;
+  wait_for_previous();
+  dependents_may_start();
 #pragma unroll
   for (int s = 0; s < G_STAGES - 1; s++) {
     if (s < steps) fill(s, kb + s * G_BK);
@@ -176,7 +178,12 @@ void launch_nt(int M, int K, const double* A, const double* B, int64_t ldb, cons
   int ks = 1;
   while (ks < 8 && nt * mt * ks * 2 <= num_sms && K >= 2 * ks * 4 * G_BK) ks *= 2;
   const int kper = ((K + ks - 1) / ks + G_BK - 1) / G_BK * G_BK;
-  const size_t smem = (size_t)G_STAGES * (G_NODES + 32 * NT) * G_BK * sizeof(double);
+  // a grid of at most one CTA per SM asks for more than half an SM's shared memory:
+  // placed early beside the kernel before it, its CTAs would pair up on the SMs
+  // that are freed first
+  const bool few = (int64_t)nt * mt * ks <= num_sms;
+  size_t smem = (size_t)G_STAGES * (G_NODES + 32 * NT) * G_BK * sizeof(double);
+  if (few) smem = std::max(smem, (size_t)120 << 10);
   auto kern = k_node_gemm64<NT>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaLaunchConfig_t cfg = {};
@@ -184,13 +191,15 @@ void launch_nt(int M, int K, const double* A, const double* B, int64_t ldb, cons
   cfg.blockDim = dim3(G_THREADS, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = ks;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = few ? 2 : 1;  // dependent (launch.hpp)
   cudaLaunchKernelEx(&cfg, kern, M, K, kper, ks, A, B, ldb, bidx, C, ldc, cidx, ncol, accumulate ? 1 : 0, sc);
 }
 

@@ -108,6 +108,8 @@ __global__ void __launch_bounds__(F_THREADS, 2)
       for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
   const int wn = (warp & 1) * 32, wm = (warp >> 1) * NT;  // the warp's first node and 8-row operator block
   const int steps = max(ce - cb, 0);
+  wait_for_previous();
+  dependents_may_start();
   if (steps > 0) fill(0, cb);
   asm volatile("cp.async.commit_group;" ::: "memory");
   for (int s = 0; s < steps; s++) {
@@ -236,7 +238,12 @@ void launch_nt(const TcOperator& A, const float* B, int64_t ldb, const int* bidx
   int ks = 1;
   while (ks < 8 && (int64_t)nt * A.ntiles * ks <= num_sms && nkt >= 4 * ks) ks *= 2;
   const int cper = (nkt + ks - 1) / ks;
-  const size_t smem = (size_t)F_STAGES * (F_NODE + 2 * 32 * NT * F_KC) * sizeof(float);
+  // a grid of at most one CTA per SM asks for more than half an SM's shared memory:
+  // placed early beside the kernel before it, its CTAs would pair up on the SMs
+  // that are freed first
+  const bool few = (int64_t)nt * A.ntiles * ks <= num_sms;
+  size_t smem = (size_t)F_STAGES * (F_NODE + 2 * 32 * NT * F_KC) * sizeof(float);
+  if (few) smem = std::max(smem, (size_t)120 << 10);
   auto kern = k_node_gemm_tf32<NT>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaLaunchConfig_t cfg = {};
@@ -244,13 +251,15 @@ void launch_nt(const TcOperator& A, const float* B, int64_t ldb, const int* bidx
   cfg.blockDim = dim3(F_THREADS, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = ks;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = few ? 2 : 1;  // dependent (launch.hpp)
   cudaLaunchKernelEx(&cfg, kern, A, cper, ks, B, ldb, bidx, C, ldc, cidx, ncol, accumulate ? 1 : 0, sc);
 }
 

@@ -407,7 +407,7 @@ __device__ __forceinline__ uint2 f16_pairs(float re, float im, float s) {
 }
 
 template <typename T, int NP>
-__global__ void __launch_bounds__(256) k_m2l_fwd_rb(M2LGeom g, const T* __restrict__ supeden,
+__global__ void __launch_bounds__(256) k_m2l_fwd_rb(M2LGeom g, const T* supeden,
                                                     const int* __restrict__ nodes, int nwork,
                                                     const int* __restrict__ depth, T* __restrict__ spectra) {
   constexpr int N = 2 * NP - 1, NH = NP, NFC = ((N * N * N + 1) / 2 + 3) / 4 * 4;
@@ -426,6 +426,8 @@ __global__ void __launch_bounds__(256) k_m2l_fwd_rb(M2LGeom g, const T* __restri
   constexpr int XL = full_lines(NP * NP), YL = full_lines(NP * NH), ZL = full_lines(N * NH);
   __shared__ Cpx<T> tw[N];
   fill_tw<T, N>(tw);
+  wait_for_previous();
+  dependents_may_start();
   const float s16 = g.sg == 2 ? spectra_scale16(g.bound) : 1.f;
   __syncthreads();
   for (int wi = blockIdx.x * wpc + warp; wi < nwork; wi += gridDim.x * wpc) {
@@ -560,7 +562,7 @@ __global__ void __launch_bounds__(256) k_m2l_fwd_rb(M2LGeom g, const T* __restri
 }
 
 template <typename T, int NP>
-__global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* __restrict__ effval,
+__global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* effval,
                                                     const int* __restrict__ work, int nwork,
                                                     T* __restrict__ tdncval) {
   constexpr int N = 2 * NP - 1, NH = NP, NFC = ((N * N * N + 1) / 2 + 3) / 4 * 4;
@@ -585,6 +587,8 @@ __global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* __restri
   Cpx<T>* Bm = reinterpret_cast<Cpx<T>*>(mine);
   Cpx<T>* A = reinterpret_cast<Cpx<T>*>(mine + align16(sizeof(Cpx<T>) * NP * N * NH));
   Cpx<T>* stage = reinterpret_cast<Cpx<T>*>(mine + inv_rb_warp_bytes<T>(NP, N, NH));
+  wait_for_previous();
+  dependents_may_start();
   __syncthreads();
   for (int wi = blockIdx.x * wpc + warp; wi < nwork; wi += gridDim.x * wpc) {
     const int node = work[wi];
@@ -739,7 +743,7 @@ void launch_m2l_forward(const M2LGeom& g, const T* supeden, const int* nodes, in
     const int gr = std::max(1, std::min((nn + w - 1) / w, 148 * 8));
     auto kern = g.np == 6 ? k_m2l_fwd_rb<T, 6> : g.np == 4 ? k_m2l_fwd_rb<T, 4> : k_m2l_fwd_rb<T, 8>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<gr, 32 * w, sm, st>>>(g, supeden, nodes, nn, depth, spectra);
+    launch_dependent(kern, gr, 32 * w, sm, st, g, supeden, nodes, nn, depth, spectra);
     return;
   }
   cudaFuncSetAttribute(k_m2l_fwd_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -775,7 +779,7 @@ void launch_m2l_inverse(const M2LGeom& g, const T* effval, const int* work, int 
     const int gr = std::max(1, std::min((nwork + w - 1) / w, 148 * 8));
     auto kern = g.np == 6 ? k_m2l_inv_rb<T, 6> : g.np == 4 ? k_m2l_inv_rb<T, 4> : k_m2l_inv_rb<T, 8>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kern<<<gr, 32 * w, sm, st>>>(g, effval, work, nwork, tdncval);
+    launch_dependent(kern, gr, 32 * w, sm, st, g, effval, work, nwork, tdncval);
     return;
   }
   cudaFuncSetAttribute(k_m2l_inv_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -205,6 +205,8 @@ void launch_sd(const double* tables, const double* spectra, size_t plane, int nf
   const size_t smem = (size_t)NF * SD * H_FRAGS * sizeof(double2);
   auto kern = k_m2l_had64<SD, NF>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // (not a dependent launch: its read-only loads of the spectra may not be moved
+  // above a wait in the kernel, and as plain loads they cost 7 % of an eval)
   kern<<<dim3((ngroup + per - 1) / per, nfc / NF, td), H_THREADS, smem, st>>>(
       reinterpret_cast<const double2*>(tables), reinterpret_cast<const double2*>(spectra), plane, nfc, ngroup, per,
       reinterpret_cast<const int2*>(g.head), g.tab, g.desc, g.out, reinterpret_cast<double2*>(effval));

@@ -98,6 +98,8 @@ __global__ void __launch_bounds__(P2P_THREADS) k_s2l(P2PArgs<T> a, const int* wo
   __shared__ Red<T, 4> red;
   __shared__ int lbeg[P2P_THREADS], pre[P2P_THREADS + 1], wsum[NSPLIT];
   __shared__ T lx[P2P_THREADS], ly[P2P_THREADS], lz[P2P_THREADS];
+  wait_for_previous();
+  dependents_may_start();
   const int w = blockIdx.x, g = work[w], tid = threadIdx.x, lane = tid & 31;
   const T rad = (T)a.radius[g];
   const double cx = a.center[3 * g], cy = a.center[3 * g + 1], cz = a.center[3 * g + 2];
@@ -295,6 +297,8 @@ __global__ void __launch_bounds__(32 * WP_WARPS)
   __shared__ WarpSrc<T> ws[WP_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpSrc<T>& w = ws[warp];
+  wait_for_previous();
+  dependents_may_start();
   const T* den = a.sden + (size_t)rhs * a.ns * SD;
   const int nt = a.nuc;
   for (int64_t wi = blockIdx.x * WP_WARPS + warp; wi < (int64_t)nwork * parts; wi += gridDim.x * WP_WARPS) {
@@ -447,6 +451,8 @@ __global__ void __launch_bounds__(32 * NWARP, sizeof(T) == 8 && KT == 111 ? 5 : 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpSrc64<T>& w = ws[warp];
   WarpSegs<T>& sgt = wg[warp];
+  wait_for_previous();
+  dependents_may_start();
   // packed FP32 Laplace sums (near field for KT 111, surfaces for MM 111)
   constexpr bool PAIR_NEAR = KT == 111 && sizeof(T) == 4, PAIR_SURF = MM == 111 && sizeof(T) == 4;
   const T* den = a.sden + (size_t)rhs * a.ns * SD;
@@ -661,8 +667,9 @@ __global__ void __launch_bounds__(32 * NWARP, sizeof(T) == 8 && KT == 111 ? 5 : 
 
 // tval of one round = the sum of its items' partial potentials, in item order
 template <typename T, int TD>
-__global__ void k_leaf_reduce(const LeafSplit* __restrict__ splits, int n, const T* __restrict__ partial,
-                              T* __restrict__ tval) {
+__global__ void k_leaf_reduce(const LeafSplit* __restrict__ splits, int n, const T* partial, T* tval) {
+  wait_for_previous();
+  dependents_may_start();
   const int e = blockIdx.x * blockDim.x + threadIdx.x, w = e / (32 * TD), k = e % (32 * TD);
   if (w >= n) return;
   const LeafSplit sp = splits[w];
@@ -676,6 +683,8 @@ __global__ void k_leaf_reduce(const LeafSplit* __restrict__ splits, int n, const
 // sden_sorted[r][i][s] = srcden[r][perm[i]][s]
 template <typename T>
 __global__ void k_scatter_den(const double* srcden, const int* perm, int ns, int sd, int nrhs, T* out) {
+  wait_for_previous();
+  dependents_may_start();
   size_t n = (size_t)ns * sd * nrhs;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     size_t r = e / ((size_t)ns * sd);
@@ -688,6 +697,8 @@ __global__ void k_scatter_den(const double* srcden, const int* perm, int ns, int
 // trgval[r][perm[i]][t] = tval[r][i][t]
 template <typename T>
 __global__ void k_gather_val(const T* tval, const int* perm, int nt, int td, int nrhs, double* trgval) {
+  wait_for_previous();
+  dependents_may_start();
   size_t n = (size_t)nt * td * nrhs;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     size_t r = e / ((size_t)nt * td);
@@ -701,6 +712,8 @@ __global__ void k_gather_val(const T* tval, const int* perm, int nt, int td, int
 // potentials plus an FP64 near-field sum
 __global__ void k_gather_val_sum(const float* tval, const double* near, const int* perm, int nt, int td, int nrhs,
                                  double* trgval) {
+  wait_for_previous();
+  dependents_may_start();
   size_t n = (size_t)nt * td * nrhs;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     size_t r = e / ((size_t)nt * td);
@@ -731,31 +744,32 @@ void launch_p2p_kt(const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cu
         const int parts = (rounds + R - 1) / R;
         const int grid = (int)std::min<int64_t>(((int64_t)w.n * parts + WP_WARPS - 1) / WP_WARPS, 148 * 32);
         if (R == 2)
-          k_s2m_warp<T, KT, 2><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+          launch_dependent(k_s2m_warp<T, KT, 2>, grid, 32 * WP_WARPS, 0, st, a, w.work, w.n, parts, rhs);
         else if (R == 5)
-          k_s2m_warp<T, KT, 5><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+          launch_dependent(k_s2m_warp<T, KT, 5>, grid, 32 * WP_WARPS, 0, st, a, w.work, w.n, parts, rhs);
         else if constexpr (sizeof(T) == 8)
-          k_s2m_warp<T, KT, 4><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+          launch_dependent(k_s2m_warp<T, KT, 4>, grid, 32 * WP_WARPS, 0, st, a, w.work, w.n, parts, rhs);
         else if (R == 10)
-          k_s2m_warp<T, KT, 10><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+          launch_dependent(k_s2m_warp<T, KT, 10>, grid, 32 * WP_WARPS, 0, st, a, w.work, w.n, parts, rhs);
         else
-          k_s2m_warp<T, KT, 16><<<grid, 32 * WP_WARPS, 0, st>>>(a, w.work, w.n, parts, rhs);
+          launch_dependent(k_s2m_warp<T, KT, 16>, grid, 32 * WP_WARPS, 0, st, a, w.work, w.n, parts, rhs);
       }
       break;
     case P2P_S2L:
       if (w.n)
-        k_s2l<T, KT><<<dim3(w.n, (a.nsurf + 31) / 32), P2P_THREADS, 0, st>>>(a, w.work, w.ptr, w.idx, rhs);
+        launch_dependent(k_s2l<T, KT>, dim3(w.n, (a.nsurf + 31) / 32), P2P_THREADS, 0, st, a, w.work, w.ptr, w.idx,
+                         rhs);
       break;
     case P2P_LEAF:
       if (w.n) {
         constexpr int nw = sizeof(T) == 4 ? 8 : 4;  // static shared memory: 64 staged sources per warp
         const int grid = std::min((w.nitem + nw - 1) / nw, 148 * 32);
-        k_leaf_warp<T, KT, nw>
-            <<<grid, 32 * nw, 0, st>>>(a, w.items, w.idx, w.idx2, w.nitem, static_cast<T*>(w.partial), rhs);
+        launch_dependent(k_leaf_warp<T, KT, nw>, grid, 32 * nw, 0, st, a, w.items, w.idx, w.idx2, w.nitem,
+                         static_cast<T*>(w.partial), rhs);
         if (w.nsplit > 0) {
           constexpr int TD = KTraits<KT>::TD;
-          k_leaf_reduce<T, TD><<<(w.nsplit * 32 * TD + 255) / 256, 256, 0, st>>>(
-              w.splits, w.nsplit, static_cast<const T*>(w.partial), a.tval + (size_t)rhs * a.nt * TD);
+          launch_dependent(k_leaf_reduce<T, TD>, (w.nsplit * 32 * TD + 255) / 256, 256, 0, st, w.splits, w.nsplit,
+                           static_cast<const T*>(w.partial), a.tval + (size_t)rhs * a.nt * TD);
         }
       }
       break;
@@ -918,7 +932,7 @@ void launch_scatter_den(const double* srcden, const int* perm, int ns, int sd, i
   size_t n = (size_t)ns * sd * nrhs;
   if (!n) return;
   int grid = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-  k_scatter_den<T><<<grid, 256, 0, st>>>(srcden, perm, ns, sd, nrhs, out);
+  launch_dependent(k_scatter_den<T>, grid, 256, 0, st, srcden, perm, ns, sd, nrhs, out);
 }
 template void launch_scatter_den<double>(const double*, const int*, int, int, int, double*, cudaStream_t);
 template void launch_scatter_den<float>(const double*, const int*, int, int, int, float*, cudaStream_t);
@@ -928,7 +942,7 @@ void launch_gather_val(const T* tval, const int* perm, int nt, int td, int nrhs,
   size_t n = (size_t)nt * td * nrhs;
   if (!n) return;
   int grid = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-  k_gather_val<T><<<grid, 256, 0, st>>>(tval, perm, nt, td, nrhs, trgval);
+  launch_dependent(k_gather_val<T>, grid, 256, 0, st, tval, perm, nt, td, nrhs, trgval);
 }
 template void launch_gather_val<double>(const double*, const int*, int, int, int, double*, cudaStream_t);
 
@@ -937,7 +951,7 @@ void launch_gather_val_sum(const float* tval, const double* near, const int* per
   size_t n = (size_t)nt * td * nrhs;
   if (!n) return;
   int grid = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-  k_gather_val_sum<<<grid, 256, 0, st>>>(tval, near, perm, nt, td, nrhs, trgval);
+  launch_dependent(k_gather_val_sum, grid, 256, 0, st, tval, near, perm, nt, td, nrhs, trgval);
 }
 template void launch_gather_val<float>(const float*, const int*, int, int, int, double*, cudaStream_t);
 
