@@ -246,7 +246,7 @@ def measured_peaks():
         return 6650.0, 1590.0, 1965.0, "fallback"
 
 
-NF6 = 4 * 6 ** 3 + 4  # stored (Hermitian-canonical) frequencies per spectrum at np=6
+NF6 = 668  # stored (Hermitian-canonical) frequencies per spectrum at np=6: (11^3 + 1) / 2, up to a multiple of 4
 NSURF6 = 6 ** 3 - 4 ** 3  # |UE| = |DC| at np=6
 # DRAM bytes (read + write) of one k_m2l_had_tc16 launch per spectrum node,
 # from an ncu capture of that kernel (dram__bytes_read.sum +
