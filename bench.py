@@ -252,7 +252,7 @@ NSURF6 = 6 ** 3 - 4 ** 3  # |UE| = |DC| at np=6
 # from an ncu capture of that kernel (dram__bytes_read.sum +
 # dram__bytes_write.sum) on the 1,048,576-point cloud of this workload,
 # scaled by the number of spectra of the workload timed here
-HAD_TRAFFIC_PER_SPECTRUM = 13665.0
+HAD_TRAFFIC_PER_SPECTRUM = 10338.0
 
 
 def roofline(phases, wc, hbm, bf16, sm_mhz, had_ms):
@@ -632,7 +632,7 @@ def engine_arm(args):
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": WORKLOAD, "n_points": n, "kernel": 111, "np": 6, "ptsmax": 64, "maxlevel": 10,
                    "precision": "mixed (FP32 point sums and spectra; V-list Hadamard on tcgen05 with FP16-pair "
-                                "operands and FP32 accumulation; surface contractions in split TF32 on tcgen05; "
+                                "operands and FP32 accumulation; surface contractions in split TF32 on the tensor cores; "
                                 "FP64 operator SVDs)", "rhs": 1,
                    "l2": "flushed (256 MB write) before every timed step", "parallelism": f"replicas x{world}"},
         "relerr": relerr, "check_targets": NCHK,
