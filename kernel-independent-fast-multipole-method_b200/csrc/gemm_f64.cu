@@ -182,10 +182,11 @@ void launch_nt(int M, int K, const double* A, const double* B, int64_t ldb, cons
   // placed early beside the kernel before it, its CTAs would pair up on the SMs
   // that are freed first
   const bool few = (int64_t)nt * mt * ks <= num_sms;
-  size_t smem = (size_t)G_STAGES * (G_NODES + 32 * NT) * G_BK * sizeof(double);
-  if (few) smem = std::max(smem, (size_t)120 << 10);
+  constexpr size_t stages = (size_t)G_STAGES * (G_NODES + 32 * NT) * G_BK * sizeof(double);
+  constexpr size_t most = std::max(stages, (size_t)120 << 10);
+  const size_t smem = few ? most : stages;
   auto kern = k_node_gemm64<NT>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);  // the same at every launch (launch.hpp)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nt * ks, mt, 1);
   cfg.blockDim = dim3(G_THREADS, 1, 1);

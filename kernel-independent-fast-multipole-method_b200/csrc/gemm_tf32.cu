@@ -242,10 +242,11 @@ void launch_nt(const TcOperator& A, const float* B, int64_t ldb, const int* bidx
   // placed early beside the kernel before it, its CTAs would pair up on the SMs
   // that are freed first
   const bool few = (int64_t)nt * A.ntiles * ks <= num_sms;
-  size_t smem = (size_t)F_STAGES * (F_NODE + 2 * 32 * NT * F_KC) * sizeof(float);
-  if (few) smem = std::max(smem, (size_t)120 << 10);
+  constexpr size_t stages = (size_t)F_STAGES * (F_NODE + 2 * 32 * NT * F_KC) * sizeof(float);
+  constexpr size_t most = std::max(stages, (size_t)120 << 10);
+  const size_t smem = few ? most : stages;
   auto kern = k_node_gemm_tf32<NT>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);  // the same at every launch (launch.hpp)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nt * ks, A.ntiles, 1);
   cfg.blockDim = dim3(F_THREADS, 1, 1);

@@ -26,6 +26,11 @@ namespace kifmm {
 // upward 1.29 -> 1.61 ms before the rule).  Measured on whole calls: Laplace np=4
 // FP64 2,000 points 126 -> 107 us, 32,768 points 308 -> 280 us, np=6 mixed 262,144
 // points 1174 -> 1110 us.
+//
+// Limits of dynamic shared memory.  cudaFuncAttributeMaxDynamicSharedMemorySize
+// belongs to the kernel, not to a launch, and handles may be evaluated by several
+// threads: a kernel whose launches differ in size sets it to its largest size
+// every time, so that no thread lowers it between another's setting and launch.
 #ifdef __CUDACC__
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

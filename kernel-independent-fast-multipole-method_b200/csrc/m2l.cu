@@ -32,6 +32,9 @@ namespace kifmm {
 namespace {
 
 constexpr int FFT_THREADS = 256;
+// shared memory of a transform CTA: the budget of its warps and, as a launch takes
+// less by np and by the layout of its spectra, every launch's limit (launch.hpp)
+constexpr size_t DFT_SMEM = 200 * 1024;
 
 template <typename T>
 struct Cpx {
@@ -729,24 +732,24 @@ template <typename T>
 void launch_m2l_forward(const M2LGeom& g, const T* supeden, const int* nodes, int nn, const int* depth, T* spectra,
                         cudaStream_t st) {
   if (nn <= 0) return;
-  // warp per node; as many warps per CTA (<= 8) as fit in ~200 KB of shared memory
+  // warp per node; as many warps per CTA (<= 8) as fit in the budget
   const size_t per_warp = fwd_warp_bytes<T>(g.np, g.n, g.nh);
   const size_t head = align16(sizeof(Cpx<T>) * g.n * g.n);
-  int wpc = (int)std::max<size_t>(1, std::min<size_t>(8, (200 * 1024 - head) / per_warp));
+  int wpc = (int)std::max<size_t>(1, std::min<size_t>(8, (DFT_SMEM - head) / per_warp));
   size_t smem = head + per_warp * wpc;
   int grid = std::max(1, std::min((nn + wpc - 1) / wpc, 148 * 8));
   if (g.np == 4 || g.np == 6 || g.np == 8) {
     const size_t head_rb = align16(sizeof(int) * g.n * g.n * g.nh);
     const size_t per_rb = fwd_rb_warp_bytes<T>(g.np, g.n, g.nh);
-    const int w = (int)std::max<size_t>(1, std::min<size_t>(8, (200 * 1024 - head_rb) / per_rb));
+    const int w = (int)std::max<size_t>(1, std::min<size_t>(8, (DFT_SMEM - head_rb) / per_rb));
     const size_t sm = head_rb + per_rb * w;
     const int gr = std::max(1, std::min((nn + w - 1) / w, 148 * 8));
     auto kern = g.np == 6 ? k_m2l_fwd_rb<T, 6> : g.np == 4 ? k_m2l_fwd_rb<T, 4> : k_m2l_fwd_rb<T, 8>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DFT_SMEM);
     launch_dependent(kern, gr, 32 * w, sm, st, g, supeden, nodes, nn, depth, spectra);
     return;
   }
-  cudaFuncSetAttribute(k_m2l_fwd_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_m2l_fwd_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DFT_SMEM);
   k_m2l_fwd_warp<T><<<grid, 32 * wpc, smem, st>>>(g, supeden, nodes, nn, depth, spectra);
 }
 
@@ -767,22 +770,22 @@ void launch_m2l_inverse(const M2LGeom& g, const T* effval, const int* work, int 
   if (nwork <= 0) return;
   const size_t per_warp = inv_warp_bytes<T>(g.np, g.n, g.nh);
   const size_t head = align16(sizeof(Cpx<T>) * g.n * g.n);
-  int wpc = (int)std::max<size_t>(1, std::min<size_t>(8, (200 * 1024 - head) / per_warp));
+  int wpc = (int)std::max<size_t>(1, std::min<size_t>(8, (DFT_SMEM - head) / per_warp));
   size_t smem = head + per_warp * wpc;
   int grid = std::max(1, std::min((nwork + wpc - 1) / wpc, 148 * 8));
   if (g.np == 4 || g.np == 6 || g.np == 8) {
     const size_t per_rb =
         inv_rb_warp_bytes<T>(g.np, g.n, g.nh) + (sizeof(T) == 4 && g.effval_sg ? inv_rb_stage_bytes<T>(g.np) : 0);
     const size_t head_rb = align16(sizeof(int) * (g.n * g.n * g.nh + g.np * g.np * g.np));
-    const int w = (int)std::max<size_t>(1, std::min<size_t>(8, (200 * 1024 - head_rb) / per_rb));
+    const int w = (int)std::max<size_t>(1, std::min<size_t>(8, (DFT_SMEM - head_rb) / per_rb));
     const size_t sm = head_rb + per_rb * w;
     const int gr = std::max(1, std::min((nwork + w - 1) / w, 148 * 8));
     auto kern = g.np == 6 ? k_m2l_inv_rb<T, 6> : g.np == 4 ? k_m2l_inv_rb<T, 4> : k_m2l_inv_rb<T, 8>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DFT_SMEM);
     launch_dependent(kern, gr, 32 * w, sm, st, g, effval, work, nwork, tdncval);
     return;
   }
-  cudaFuncSetAttribute(k_m2l_inv_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_m2l_inv_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DFT_SMEM);
   k_m2l_inv_warp<T><<<grid, 32 * wpc, smem, st>>>(g, effval, work, nwork, tdncval);
 }
 

@@ -655,7 +655,8 @@ void had_tc16_launch_g(const unsigned char* img, const unsigned* spectra, int nq
   const int grid = std::min(num_sms, nitems);
   const size_t smem = h16_smem(H16Shape<TD>::IMGB, (nitems + grid - 1) / grid);
   auto kern = k_m2l_had_tc16<NF, G, SD, TD>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // 227 KB a CTA less the kernel's static 1,024 bytes: the launches' sizes vary with the tree (launch.hpp)
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
   kern<<<grid, h16_threads(G), smem, st>>>(img, spectra, nq, ntiles, qchd, ctab, tile_dirs, effval, nitems, plane,
                                            bound, inv_sb, wait_limit, status);
 }
