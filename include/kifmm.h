@@ -163,7 +163,8 @@ kifmm_status kifmm_direct(kifmm_handle h, const double* srcden, int nt, const do
  * whose GPU memory is owned by a framework's caching allocator or a fixed
  * budget reserved at start-up cannot call cudaMalloc between its steps.
  * All pointers are device pointers the caller allocated (layouts as in
- * kifmm_direct); the work is enqueued on `stream` (NULL = legacy default
+ * kifmm_direct; d_trgval is written after every input has been read, so it
+ * may be one of them); the work is enqueued on `stream` (NULL = legacy default
  * stream) and the call does not synchronise.  The call allocates nothing:
  * its partial sums live in one fixed device array of
  * KIFMM_NOALLOC_SCRATCH_DOUBLES doubles (8 MiB, held on every GPU that loads

@@ -162,7 +162,8 @@ void launch_direct(int kt, const DirectPlan& p, const double* spos, const double
                    cudaStream_t st) {
   if (nt <= 0) return;
   const KConst<double> kc{kc3[0], kc3[1], kc3[2]};
-  double* partial = p.nchunk > 1 ? scratch : out;
+  const bool staged = p.nchunk > 1 || p.staged;
+  double* partial = staged ? scratch : out;
   int td = 1;
   switch (kt) {
     case 111: launch_partial_g<111>(p, spos, snor, sden, ns, tpos, nt, partial, kc, st); break;
@@ -175,7 +176,7 @@ void launch_direct(int kt, const DirectPlan& p, const double* spos, const double
     case 521: launch_partial_g<521>(p, spos, snor, sden, ns, tpos, nt, partial, kc, st); td = 3; break;
     default: return;
   }
-  if (p.nchunk > 1) {
+  if (staged) {
     const size_t n = (size_t)nt * td;
     const int grid = (int)std::min<size_t>((n + 31) / 32, (size_t)num_sms * 8);
     k_direct_reduce<<<std::max(1, grid), 256, 0, st>>>(partial, p.nchunk, n, out);

@@ -114,9 +114,12 @@ void launch_p2p(int kt, const P2PArgs<T>& a, const P2PWork& w, int which, int rh
 
 // Direct sum (direct.cu): the split of the sources into chunks, whose partial
 // potentials take `scratch` doubles (0: one chunk, written straight to out).
+// staged: one chunk takes nt * td doubles of scratch too, so that out is written
+// only once every input has been read and may be one of the inputs.
 struct DirectPlan {
   int G = 128, tblocks = 0, nchunk = 1, chunk = 1;
   size_t scratch = 0;
+  bool staged = false;
 };
 DirectPlan direct_plan(int ns, int nt, int td, int num_sms, size_t capacity);
 // snor is read for double-layer kernels only

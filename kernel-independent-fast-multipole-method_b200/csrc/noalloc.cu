@@ -13,7 +13,8 @@
 // How: the sources are split into chunks evaluated by different CTAs (so a
 // small target set still fills the GPU, direct.cu); each chunk's partial potentials go
 // to a fixed scratch array in device global memory, declared below at file
-// scope, and a second kernel adds the chunks up into the caller's output.
+// scope, and a second kernel adds the chunks up into the caller's output, which
+// may therefore be one of the inputs.
 // The scratch holds KIFMM_NOALLOC_SCRATCH_DOUBLES doubles (8 MiB) on every
 // GPU that loads this library, for the life of the process.  A call needs
 // nchunk * nt * tdof of them; nt * tdof above the capacity is rejected with
@@ -80,7 +81,8 @@ extern "C" kifmm_status kifmm_direct_noalloc(int kt, int ncoef, const double* co
   double kcd[3], cf[2] = {1.0, 0.25};
   for (int i = 0; i < ncoef && i < 2; i++) cf[i] = coefs[i];
   kernel_constants(kt, cf, kcd);
-  const DirectPlan plan = direct_plan(ns, nt, td, num_sms, (size_t)KIFMM_NOALLOC_SCRATCH_DOUBLES);
+  DirectPlan plan = direct_plan(ns, nt, td, num_sms, (size_t)KIFMM_NOALLOC_SCRATCH_DOUBLES);
+  plan.staged = true;  // the caller's output may be one of its inputs
   launch_direct(kt, plan, d_srcpos, d_srcnor, d_srcden, ns, d_trgpos, nt, d_trgval, scratch, kcd, num_sms, st);
   if (cudaGetLastError() != cudaSuccess) return KIFMM_ERR_CUDA;
   return KIFMM_OK;

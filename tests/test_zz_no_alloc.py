@@ -100,3 +100,22 @@ def test_request_beyond_the_fixed_scratch_is_refused(gpu):
     st = L.kifmm_direct_noalloc(311, 2, cf.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), 10, one, one, one, nt,
                                 one, one, None)
     assert st == kifmm.KIFMM_ERR_CAPACITY
+
+
+@pytest.mark.parametrize("kt,n", [(111, 40), (111, 128), (311, 100), (111, 6000)])
+def test_output_may_be_the_density_array(gpu, kt, n):
+    """Potentials written over the densities they come from (one chunk of
+    sources and many): every source is read before any target is written."""
+    torch = pytest.importorskip("torch")
+    src, nor, den, _ = case(kt, n, 10, n)
+    cf = np.array([1.0, 0.25])
+    dev = lambda a: torch.tensor(np.ascontiguousarray(a, np.float64).reshape(-1), device="cuda")
+    d_src, d_nor, d_den = dev(src), dev(nor), dev(den)
+    stream = torch.cuda.current_stream()
+    st = kifmm.lib().kifmm_direct_noalloc(kt, 2, cf.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), n,
+                                          d_src.data_ptr(), d_nor.data_ptr(), d_den.data_ptr(), n, d_src.data_ptr(),
+                                          d_den.data_ptr(), stream.cuda_stream)
+    assert st == kifmm.KIFMM_OK, kifmm.STATUS.get(st, st)
+    stream.synchronize()
+    ref = existing_direct(kt, cf, src, nor, den, src)
+    assert np.linalg.norm(d_den.cpu().numpy() - ref) <= TOL * np.linalg.norm(ref)
