@@ -36,9 +36,10 @@ struct Red {
 };
 
 // Packed staged source: (x, y, z, first density component); a single-dof
-// single-layer interaction then reads one 16-byte (FP32) word.
+// single-layer interaction then reads one 16-byte (FP32) word, and lap_pairs a
+// pair of sources as two of them.
 template <typename T>
-struct P4 {
+struct alignas(16) P4 {
   T x, y, z, w;
 };
 
@@ -232,6 +233,7 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 // (the 1e-16 cut-off as in keval), for two targets t_k = (px, py, pz)[k]
 __device__ __forceinline__ void lap_pairs(const WarpSrc64<float>& w, const float* px, const float* py,
                                           const float* pz, int sg, int nsplit, int npairs, float* s) {
+  static_assert(alignof(WarpSrc64<float>) % alignof(float4) == 0, "16-byte loads of the staged sources");
   const float4* wp = reinterpret_cast<const float4*>(w.p);
   unsigned long long PX[2], PY[2], PZ[2], S[2];
 #pragma unroll
