@@ -41,20 +41,24 @@ struct KConst {
 __device__ __forceinline__ float fmt(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fmt(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// FP32: the hardware approximation with denormal inputs flushed (every caller
-// has r^2 >= 1e-16), which drops the denormal rescaling steps of rsqrtf
+// FP32: the approximate reciprocal root of the instruction set; every caller
+// has r^2 >= 1e-16, so subnormal inputs, which it flushes, do not occur
 __device__ __forceinline__ float rsqrt_t(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// FP64: the approximate reciprocal root (rsqrt.approx.ftz.f64, 9.3e-7 measured)
-// and one step of Householder's third-order iteration on it, with the residual
-// e = 1 - x y^2: y (1 + e/2 + 3 e^2 / 8), error 5 e^3 / 16 < 3e-18.  For
-// normal, finite x; within one unit in the last place of rsqrt() over
-// [1e-16, 1e2].  Five FP64 instructions and no special-case branch
-// (dependent chains of each, 148 SMs: 2.55e12 per second, rsqrt() 1.75e12);
-// the FP64 pipe (64 lanes per SM and clock) bounds every FP64 sum.
+// FP64, for normal finite x: an approximate root y and one correction.  With
+// the residual e = 1 - x y^2 the root is exactly y (1 - e)^(-1/2), whose binomial
+// series is y (1 + e/2 + 3 e^2/8 + 5 e^3/16 + ...); stopping at e^2 is Chebyshev's
+// third-order iteration for y^-2 - x = 0 (J. F. Traub, Iterative Methods for the
+// Solution of Equations, 1964, basic sequence E_3).  The seed is within 1e-6
+// (9.3e-7 measured), so |e| < 2.1e-6 and the first dropped term is below 3e-18;
+// rounding x y moves the result by at most half a unit in the last place and
+// the last operation by another: 1.03 units in all (tests/test_gpu_root.py, from
+// 1e-16 to the largest number).  Five FP64 instructions beside the seed; the
+// FP64 pipe (64 lanes per SM and clock) bounds every FP64 sum (dependent
+// chains, 148 SMs: 2.55e12 roots per second, with rsqrt() 1.75e12).
 __device__ __forceinline__ double rsqrt_t(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -64,8 +68,8 @@ __device__ __forceinline__ double rsqrt_t(double x) {
 
 // 1/r from r^2, 0 below the cut-off r^2 < 1e-16
 __device__ __forceinline__ float rinv_cut(float r2) { return (r2 >= 1e-16f) ? rsqrt_t(r2) : 0.f; }
-// FP64: the cut-off, an infinite and a NaN r^2 (1/r = 0, as from rsqrt() and
-// from the failed comparison) in one unsigned range test of the bit pattern,
+// FP64: the cut-off, an infinite r^2 and a NaN (1/r = 0 in FP32 too, from the root
+// of infinity and from the failed comparison) in one unsigned range test of the bit pattern,
 // which leaves the FP64 pipe to the sum
 __device__ __forceinline__ double rinv_cut(double r2) {
   constexpr unsigned long long lo = 0x3C9CD2B297D889BCull;  // 1e-16

@@ -1,4 +1,6 @@
+import ctypes
 import os
+import subprocess
 import sys
 
 import pytest
@@ -27,3 +29,16 @@ def gpu():
     if not has_gpu():
         pytest.skip("no CUDA device")
     return True
+
+
+@pytest.fixture(scope="session")
+def harness(tmp_path_factory):
+    """tests/device_harness.cu, compiled beside the built library."""
+    out = str(tmp_path_factory.mktemp("harness") / "libharness.so")
+    lib = os.path.join(PKG, "lib")
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    subprocess.run([nvcc, "-std=c++17", "-O2", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler",
+                    "-fPIC", "-cudart", "shared", "-I", os.path.join(PKG, "csrc"), "-o", out,
+                    os.path.join(ROOT, "tests", "device_harness.cu"), "-L", lib, "-lkifmm_b200", "-Xlinker",
+                    "-rpath," + lib], check=True)
+    return ctypes.CDLL(out)
