@@ -428,9 +428,12 @@ __global__ void __launch_bounds__(32 * WP_WARPS)
 // bisection of the warp's prefix sums), then the W-list upward equivalent
 // surfaces and the leaf's own downward equivalent surface.  An item of a cut
 // range writes partial[out][slot][d] (T, the accumulator's type), which
-// k_leaf_reduce adds up in item order.  The register limits (64 in FP32, 128 and
-// for FP64 Laplace 96) let 32, 16 and 20 warps share an SM, which hides the staging
-// loads: FP32 2.39 -> 2.26 ms at 4M points against the compiler's own 80.
+// k_leaf_reduce adds up in item order.  Limits on the registers trade spills for
+// warps, whose number hides the staging loads.  FP32: 64 registers (32 warps an
+// SM) for the scalar single layers, 80 (24 warps) for the others, which spill at
+// 64; leaf pass of 262,144 Laplace points 0.261 ms with 64, 0.263 with 80 and 0.327
+// with 108, of 100,003 Stokes points 0.134, 0.126 and 0.142, of as many Navier points
+// 0.132, 0.125 and 0.136.  FP64: 128, and for Laplace 96 (16 and 20 warps).
 template <typename T>
 struct WarpSegs {
   int beg[32];
@@ -440,10 +443,17 @@ struct WarpSegs {
   const T* den[32];
 };
 
+// CTAs per SM that the registers are limited for (comment above)
+template <typename T, int KT>
+constexpr int leaf_ctas() {
+  if (sizeof(T) == 8) return KT == 111 ? 5 : 4;
+  return KTraits<KT>::TD == 1 && !KTraits<KT>::DL ? 4 : 3;
+}
+
 template <typename T, int KT, int NWARP>
-__global__ void __launch_bounds__(32 * NWARP, sizeof(T) == 8 && KT == 111 ? 5 : 4) k_leaf_warp(P2PArgs<T> a, const LeafItem* __restrict__ items,
-                                                          const int* __restrict__ nidx, const int* __restrict__ midx,
-                                                          int nitem, T* __restrict__ partial, int rhs) {
+__global__ void __launch_bounds__(32 * NWARP, leaf_ctas<T, KT>())
+    k_leaf_warp(P2PArgs<T> a, const LeafItem* __restrict__ items, const int* __restrict__ nidx,
+                const int* __restrict__ midx, int nitem, T* __restrict__ partial, int rhs) {
   constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD;
   constexpr bool DL = KTraits<KT>::DL;
   constexpr int MM = KTraits<KT>::MM;
