@@ -443,6 +443,13 @@ struct WarpSegs {
   const T* den[32];
 };
 
+// target slots of a round with `left` targets to go, two targets each
+__host__ __device__ inline int leaf_slots(int left) {
+  int G = 1;
+  while (2 * G < left && G < 16) G <<= 1;
+  return G;
+}
+
 // CTAs per SM that the registers are limited for (comment above)
 template <typename T, int KT>
 constexpr int leaf_ctas() {
@@ -480,8 +487,7 @@ __global__ void __launch_bounds__(32 * NWARP, leaf_ctas<T, KT>())
     const int nsurf_segs = it.nm + it.l2t;
     int left = it.take;  // point sources of this item still to come
     {
-      int G = 1;
-      while (2 * G < nt - it.tb && G < 16) G <<= 1;
+      const int G = leaf_slots(nt - it.tb);
       const int nsplit = 32 / G, slot = lane % G, sg = lane / G;
       bool valid[2];  // targets it.tb + slot and it.tb + slot + G
       T px[2], py[2], pz[2], acc[2][TD];
@@ -791,18 +797,21 @@ void launch_p2p_kt(const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cu
 }  // namespace
 
 namespace {
+// evaluations per lane of `all` sources at a round's targets: 32 / slots lanes
+// share a source's two targets, a round of one target computes its second in vain
+double leaf_cost(int64_t all, int left) { return (double)all * leaf_slots(left) / 16; }
+
 // the items of leaves w0 .. w1 - 1 of leaf_items, partial rows counted from 0
-template <class Lanes>
 void cut_leaves(int w0, int w1, const int* work, const int* tcnt, const int* scnt, const int64_t* nptr, const int* nidx,
                 const int64_t* mptr, const unsigned char* l2t, const int* tbeg, int nsurf, double limit,
-                const int64_t* nsrc, Lanes lanes, std::vector<LeafItem>* items, std::vector<LeafSplit>* splits,
+                const int64_t* nsrc, std::vector<LeafItem>* items, std::vector<LeafSplit>* splits,
                 int* nparts) {
   for (int w = w0; w < w1; w++) {
     const int g = work[w], nt = tcnt[g];
     const int nseg = (int)(mptr[w + 1] - mptr[w]) + l2t[w];
     const int64_t all = nsrc[w] + (int64_t)nseg * nsurf;
     for (int tb = 0; tb < nt; tb += 32) {
-      const double cost = (double)all / lanes(nt - tb);
+      const double cost = leaf_cost(all, nt - tb);
       const int parts = cost > 1.5 * limit ? (int)std::min(cost / limit + 0.5, 65536.0) : 1;
       int64_t seg = nptr[w];  // the near segment the next item begins in, `skip` sources into it
       int skip = 0, s0 = 0;   // and its first surface
@@ -863,19 +872,16 @@ void cut_leaves(int w0, int w1, const int* work, const int* tcnt, const int* scn
 // leaf with long lists to one warp (150,001 sources on an ellipsoid, targets
 // in the volume: the coarse leaves' W lists hold hundreds of surfaces, 17.9 ms
 // in that warp's tail) and a small tree's leaves on a few SMs (2,000 points:
-// 56 warps, 0.15 ms).  A range costs its sources over the lanes that share a
-// target; it is cut above `limit` = 1/8 of a warp's share when every SM holds
-// 32 warps, and not below `least` sources (two staged batches in FP64, four in
-// FP32, whose pairs take a quarter of the time), where starting an item and
-// adding its partial sum would cost more than the sources.
+// 56 warps, 0.15 ms).  A range costs its evaluations per lane (leaf_cost; with a
+// round of one target counted at half of that, 150,001 ellipsoid sources to 5,000
+// volume targets took 0.167 ms instead of 0.122); it is cut above `limit` = 1/8 of
+// a warp's share when every SM holds 32 warps, and not below `least` sources
+// (two staged batches in FP64, four in FP32, whose pairs take a quarter of the
+// time), where starting an item and adding its partial sum would cost more than
+// the sources.
 void leaf_items(int nwork, const int* work, const int* tcnt, const int* scnt, const int64_t* nptr, const int* nidx,
                 const int64_t* mptr, const unsigned char* l2t, const int* tbeg, int nsurf, int least, int num_sms,
                 std::vector<LeafItem>* items, std::vector<LeafSplit>* splits, int* nparts) {
-  auto lanes = [](int left) {  // lanes that share a target in a round with `left` targets to go
-    int G = 1;
-    while (G < left && G < 32) G <<= 1;
-    return 32 / G;
-  };
   // the leaves in contiguous ranges, one host thread each
   const int nthr = host_parallel_threads(nwork / 2048);
   auto run = [&](auto&& body) {  // body(t, first leaf, past the last)
@@ -892,8 +898,8 @@ void leaf_items(int nwork, const int* work, const int* tcnt, const int* scnt, co
       for (int64_t k = nptr[w]; k < nptr[w + 1]; k++) s += scnt[nidx[k]];
       nsrc[w] = s;
       const int nt = tcnt[work[w]];
-      const double all = (double)s + (double)nsurf * ((mptr[w + 1] - mptr[w]) + l2t[w]);
-      for (int tb = 0; tb < nt; tb += 32) total += all / lanes(nt - tb);
+      const int64_t all = s + (mptr[w + 1] - mptr[w] + l2t[w]) * nsurf;
+      for (int tb = 0; tb < nt; tb += 32) total += leaf_cost(all, nt - tb);
     }
     totals[t] = total;
   });
@@ -904,8 +910,8 @@ void leaf_items(int nwork, const int* work, const int* tcnt, const int* scnt, co
   std::vector<std::vector<LeafSplit>> psplits(nthr);
   std::vector<int> pparts(nthr, 0);
   run([&](int t, int w0, int w1) {
-    cut_leaves(w0, w1, work, tcnt, scnt, nptr, nidx, mptr, l2t, tbeg, nsurf, limit, nsrc.data(), lanes, &pitems[t],
-               &psplits[t], &pparts[t]);
+    cut_leaves(w0, w1, work, tcnt, scnt, nptr, nidx, mptr, l2t, tbeg, nsurf, limit, nsrc.data(), &pitems[t], &psplits[t],
+               &pparts[t]);
   });
   items->clear();
   splits->clear();
