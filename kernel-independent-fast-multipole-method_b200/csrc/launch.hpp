@@ -18,10 +18,11 @@ namespace kifmm {
 // called dependents_may_start(), and must call wait_for_previous() before it
 // touches anything an earlier kernel of the stream writes or reads: the call
 // returns when the kernel before has completed and its writes are visible.
-// Every kernel of the chain waits, so completion is transitive.  What an earlier
-// kernel writes is read through plain pointers: the compiler may move read-only
-// loads (const __restrict__, __ldg) above the wait.  A grid between one CTA
-// per SM and many waves is launched normally: started early, its CTAs pair up on
+// Every kernel of the chain waits, so completion is transitive.  What another
+// kernel of the chain writes or reads is accessed through pointers without
+// __restrict__ (and without __ldg): the compiler may take such memory for
+// untouched by the wait and move accesses above it.  Set-up data may be qualified.
+// A grid between one CTA per SM and many waves is launched normally: started early, its CTAs pair up on
 // the SMs that the kernel before frees first (FP64 contractions of Stokes np=6:
 // upward 1.29 -> 1.61 ms before the rule).  Measured on whole calls: Laplace np=4
 // FP64 2,000 points 126 -> 107 us, 32,768 points 308 -> 280 us, np=6 mixed 262,144
@@ -31,6 +32,7 @@ namespace kifmm {
 // belongs to the kernel, not to a launch, and handles may be evaluated by several
 // threads: a kernel whose launches differ in size sets it to its largest size
 // every time, so that no thread lowers it between another's setting and launch.
+constexpr int B200_SMS = 148;
 #ifdef __CUDACC__
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -46,7 +48,7 @@ inline void launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t s
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   const long long ctas = (long long)grid.x * grid.y * grid.z;
-  cfg.numAttrs = ctas <= 148 || ctas >= 148 * 16 ? 1 : 0;
+  cfg.numAttrs = ctas <= B200_SMS || ctas >= B200_SMS * 16 ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 #endif

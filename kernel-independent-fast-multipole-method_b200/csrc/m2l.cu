@@ -412,7 +412,7 @@ __device__ __forceinline__ uint2 f16_pairs(float re, float im, float s) {
 template <typename T, int NP>
 __global__ void __launch_bounds__(256) k_m2l_fwd_rb(M2LGeom g, const T* supeden,
                                                     const int* __restrict__ nodes, int nwork,
-                                                    const int* __restrict__ depth, T* __restrict__ spectra) {
+                                                    const int* __restrict__ depth, T* spectra) {
   constexpr int N = 2 * NP - 1, NH = NP, NFC = ((N * N * N + 1) / 2 + 3) / 4 * 4;
   constexpr int NSURF = NP * NP * NP - (NP - 2) * (NP - 2) * (NP - 2);
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(256) k_m2l_fwd_rb(M2LGeom g, const T* supeden,
 template <typename T, int NP>
 __global__ void __launch_bounds__(256) k_m2l_inv_rb(M2LGeom g, const T* effval,
                                                     const int* __restrict__ work, int nwork,
-                                                    T* __restrict__ tdncval) {
+                                                    T* tdncval) {
   constexpr int N = 2 * NP - 1, NH = NP, NFC = ((N * N * N + 1) / 2 + 3) / 4 * 4;
   constexpr int NSURF = NP * NP * NP - (NP - 2) * (NP - 2) * (NP - 2);
   constexpr int XL = full_lines(NP * NP), YL = full_lines(NP * NH), ZL = full_lines(N * NH);
@@ -737,13 +737,13 @@ void launch_m2l_forward(const M2LGeom& g, const T* supeden, const int* nodes, in
   const size_t head = align16(sizeof(Cpx<T>) * g.n * g.n);
   int wpc = (int)std::max<size_t>(1, std::min<size_t>(8, (DFT_SMEM - head) / per_warp));
   size_t smem = head + per_warp * wpc;
-  int grid = std::max(1, std::min((nn + wpc - 1) / wpc, 148 * 8));
+  int grid = std::max(1, std::min((nn + wpc - 1) / wpc, B200_SMS * 8));
   if (g.np == 4 || g.np == 6 || g.np == 8) {
     const size_t head_rb = align16(sizeof(int) * g.n * g.n * g.nh);
     const size_t per_rb = fwd_rb_warp_bytes<T>(g.np, g.n, g.nh);
     const int w = (int)std::max<size_t>(1, std::min<size_t>(8, (DFT_SMEM - head_rb) / per_rb));
     const size_t sm = head_rb + per_rb * w;
-    const int gr = std::max(1, std::min((nn + w - 1) / w, 148 * 8));
+    const int gr = std::max(1, std::min((nn + w - 1) / w, B200_SMS * 8));
     auto kern = g.np == 6 ? k_m2l_fwd_rb<T, 6> : g.np == 4 ? k_m2l_fwd_rb<T, 4> : k_m2l_fwd_rb<T, 8>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DFT_SMEM);
     launch_dependent(kern, gr, 32 * w, sm, st, g, supeden, nodes, nn, depth, spectra);
@@ -772,14 +772,14 @@ void launch_m2l_inverse(const M2LGeom& g, const T* effval, const int* work, int 
   const size_t head = align16(sizeof(Cpx<T>) * g.n * g.n);
   int wpc = (int)std::max<size_t>(1, std::min<size_t>(8, (DFT_SMEM - head) / per_warp));
   size_t smem = head + per_warp * wpc;
-  int grid = std::max(1, std::min((nwork + wpc - 1) / wpc, 148 * 8));
+  int grid = std::max(1, std::min((nwork + wpc - 1) / wpc, B200_SMS * 8));
   if (g.np == 4 || g.np == 6 || g.np == 8) {
     const size_t per_rb =
         inv_rb_warp_bytes<T>(g.np, g.n, g.nh) + (sizeof(T) == 4 && g.effval_sg ? inv_rb_stage_bytes<T>(g.np) : 0);
     const size_t head_rb = align16(sizeof(int) * (g.n * g.n * g.nh + g.np * g.np * g.np));
     const int w = (int)std::max<size_t>(1, std::min<size_t>(8, (DFT_SMEM - head_rb) / per_rb));
     const size_t sm = head_rb + per_rb * w;
-    const int gr = std::max(1, std::min((nwork + w - 1) / w, 148 * 8));
+    const int gr = std::max(1, std::min((nwork + w - 1) / w, B200_SMS * 8));
     auto kern = g.np == 6 ? k_m2l_inv_rb<T, 6> : g.np == 4 ? k_m2l_inv_rb<T, 4> : k_m2l_inv_rb<T, 8>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DFT_SMEM);
     launch_dependent(kern, gr, 32 * w, sm, st, g, effval, work, nwork, tdncval);

@@ -460,7 +460,7 @@ constexpr int leaf_ctas() {
 template <typename T, int KT, int NWARP>
 __global__ void __launch_bounds__(32 * NWARP, leaf_ctas<T, KT>())
     k_leaf_warp(P2PArgs<T> a, const LeafItem* __restrict__ items, const int* __restrict__ nidx,
-                const int* __restrict__ midx, int nitem, T* __restrict__ partial, int rhs) {
+                const int* __restrict__ midx, int nitem, T* partial, int rhs) {
   constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD;
   constexpr bool DL = KTraits<KT>::DL;
   constexpr int MM = KTraits<KT>::MM;
@@ -753,14 +753,14 @@ void launch_p2p_kt(const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cu
         // one warp's rounds do not set the time, and for other np.
         const int rounds = (a.nuc + 31) / 32;
         int R = 2;
-        if (w.n >= 148 * 32) {
+        if (w.n >= B200_SMS * 32) {
           if (sizeof(T) == 8)
             R = rounds % 5 == 0 ? 5 : rounds % 4 == 0 ? 4 : 2;
           else if (rounds == 5 || rounds == 10 || rounds == 16)
             R = rounds;
         }
         const int parts = (rounds + R - 1) / R;
-        const int grid = (int)std::min<int64_t>(((int64_t)w.n * parts + WP_WARPS - 1) / WP_WARPS, 148 * 32);
+        const int grid = (int)std::min<int64_t>(((int64_t)w.n * parts + WP_WARPS - 1) / WP_WARPS, B200_SMS * 32);
         if (R == 2)
           launch_dependent(k_s2m_warp<T, KT, 2>, grid, 32 * WP_WARPS, 0, st, a, w.work, w.n, parts, rhs);
         else if (R == 5)
@@ -781,7 +781,7 @@ void launch_p2p_kt(const P2PArgs<T>& a, const P2PWork& w, int which, int rhs, cu
     case P2P_LEAF:
       if (w.n) {
         constexpr int nw = sizeof(T) == 4 ? 8 : 4;  // static shared memory: 64 staged sources per warp
-        const int grid = std::min((w.nitem + nw - 1) / nw, 148 * 32);
+        const int grid = std::min((w.nitem + nw - 1) / nw, B200_SMS * 32);
         launch_dependent(k_leaf_warp<T, KT, nw>, grid, 32 * nw, 0, st, a, w.items, w.idx, w.idx2, w.nitem,
                          static_cast<T*>(w.partial), rhs);
         if (w.nsplit > 0) {
@@ -949,7 +949,7 @@ template <typename T>
 void launch_scatter_den(const double* srcden, const int* perm, int ns, int sd, int nrhs, T* out, cudaStream_t st) {
   size_t n = (size_t)ns * sd * nrhs;
   if (!n) return;
-  int grid = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
+  int grid = (int)std::min<size_t>((n + 255) / 256, B200_SMS * 16);
   launch_dependent(k_scatter_den<T>, grid, 256, 0, st, srcden, perm, ns, sd, nrhs, out);
 }
 template void launch_scatter_den<double>(const double*, const int*, int, int, int, double*, cudaStream_t);
@@ -959,7 +959,7 @@ template <typename T>
 void launch_gather_val(const T* tval, const int* perm, int nt, int td, int nrhs, double* trgval, cudaStream_t st) {
   size_t n = (size_t)nt * td * nrhs;
   if (!n) return;
-  int grid = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
+  int grid = (int)std::min<size_t>((n + 255) / 256, B200_SMS * 16);
   launch_dependent(k_gather_val<T>, grid, 256, 0, st, tval, perm, nt, td, nrhs, trgval);
 }
 template void launch_gather_val<double>(const double*, const int*, int, int, int, double*, cudaStream_t);
@@ -968,7 +968,7 @@ void launch_gather_val_sum(const float* tval, const double* near, const int* per
                            double* trgval, cudaStream_t st) {
   size_t n = (size_t)nt * td * nrhs;
   if (!n) return;
-  int grid = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
+  int grid = (int)std::min<size_t>((n + 255) / 256, B200_SMS * 16);
   launch_dependent(k_gather_val_sum, grid, 256, 0, st, tval, near, perm, nt, td, nrhs, trgval);
 }
 template void launch_gather_val<float>(const float*, const int*, int, int, int, double*, cudaStream_t);
