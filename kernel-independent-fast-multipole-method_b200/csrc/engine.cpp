@@ -339,7 +339,6 @@ struct Impl : ImplBase {
     args.tbeg = upload(tr.tbeg);
     args.tcnt = upload(tr.tcnt);
     d_depth = upload(tr.depth);
-    args.depth = d_depth;
     d_path = upload(tr.path);
     args.center = upload(tr.center);
     args.radius = upload(tr.radius);
@@ -386,7 +385,6 @@ struct Impl : ImplBase {
       a64.scnt = args.scnt;
       a64.tbeg = args.tbeg;
       a64.tcnt = args.tcnt;
-      a64.depth = args.depth;
       a64.center = args.center;
       a64.radius = args.radius;
       a64.sx = upload(sl[0]);

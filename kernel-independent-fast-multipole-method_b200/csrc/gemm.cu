@@ -37,14 +37,13 @@ __device__ __forceinline__ double row_scale(const GemmScale& sc, int j, int r) {
 }
 
 // partial != nullptr: write the unscaled K-slice sums to partial[z][j][r].
-template <typename T>
-__global__ void __launch_bounds__(NTH) k_node_gemm(int M, int K, int kchunk, const T* __restrict__ A,
-                                                   const T* __restrict__ B, int64_t ldb, const int* __restrict__ bidx,
-                                                   T* __restrict__ C, int64_t ldc, const int* __restrict__ cidx,
+__global__ void __launch_bounds__(NTH) k_node_gemm(int M, int K, int kchunk, const float* __restrict__ A,
+                                                   const float* __restrict__ B, int64_t ldb, const int* __restrict__ bidx,
+                                                   float* __restrict__ C, int64_t ldc, const int* __restrict__ cidx,
                                                    int ncol, int accumulate, GemmScale sc,
                                                    double* __restrict__ partial) {
-  __shared__ T As[BK][BM + 1];
-  __shared__ T Bs[BK][BN + 1];
+  __shared__ float As[BK][BM + 1];
+  __shared__ float Bs[BK][BN + 1];
   __shared__ int64_t bcol[BN], ccol[BN];
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BM;
@@ -56,29 +55,29 @@ __global__ void __launch_bounds__(NTH) k_node_gemm(int M, int K, int kchunk, con
     ccol[tid] = (j < ncol) ? (int64_t)cidx[j] * ldc : -1;
   }
   const int tx = tid % 16, ty = tid / 16;
-  T acc[4][4];
+  float acc[4][4];
 #pragma unroll
   for (int i = 0; i < 4; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = T(0);
+    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
   __syncthreads();
   for (int k0 = kb; k0 < ke; k0 += BK) {
     for (int e = tid; e < BM * BK; e += NTH) {
       int r = e / BK, c = e % BK;
       int gr = m0 + r, gc = k0 + c;
-      As[c][r] = (gr < M && gc < ke) ? A[(size_t)gr * K + gc] : T(0);
+      As[c][r] = (gr < M && gc < ke) ? A[(size_t)gr * K + gc] : 0.f;
     }
     for (int e = tid; e < BN * BK; e += NTH) {
       int j = e / BK, c = e % BK;
       int gc = k0 + c;
-      T v = T(0);
+      float v = 0.f;
       if (bcol[j] >= 0 && gc < ke) v = B[bcol[j] + gc];
       Bs[c][j] = v;
     }
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
-      T a[4], b[4];
+      float a[4], b[4];
 #pragma unroll
       for (int i = 0; i < 4; i++) a[i] = As[kk][ty + 16 * i];
 #pragma unroll
@@ -103,27 +102,26 @@ __global__ void __launch_bounds__(NTH) k_node_gemm(int M, int K, int kchunk, con
         partial[((size_t)blockIdx.z * ncol + col) * M + r] = (double)acc[i][j];
         continue;
       }
-      T* p = C + ccol[jj] + r;
+      float* p = C + ccol[jj] + r;
       double v = (double)acc[i][j] * row_scale(sc, col, r);
       if (accumulate) v += (double)*p;
-      *p = (T)v;
+      *p = (float)v;
     }
   }
 }
 
-template <typename T>
 __global__ void k_node_gemm_reduce(int M, int ncol, int nslice, const double* __restrict__ partial,
-                                   T* __restrict__ C, int64_t ldc, const int* __restrict__ cidx, int accumulate,
+                                   float* __restrict__ C, int64_t ldc, const int* __restrict__ cidx, int accumulate,
                                    GemmScale sc) {
   const size_t n = (size_t)ncol * M;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     int col = (int)(e / M), r = (int)(e % M);
     double s = 0.0;
     for (int z = 0; z < nslice; z++) s += partial[(size_t)z * n + e];
-    T* p = C + (int64_t)cidx[col] * ldc + r;
+    float* p = C + (int64_t)cidx[col] * ldc + r;
     double v = s * row_scale(sc, col, r);
     if (accumulate) v += (double)*p;
-    *p = (T)v;
+    *p = (float)v;
   }
 }
 
@@ -131,7 +129,7 @@ __global__ void k_node_gemm_reduce(int M, int ncol, int nslice, const double* __
 
 int launch_node_gemm(int M, int K, const float* A, const float* B, int64_t ldb, const int* bidx, float* C, int64_t ldc,
                      const int* cidx, int ncol, bool accumulate, const GemmScale& sc, double* ws, size_t ws_len,
-                      int num_sms, cudaStream_t st) {
+                     int num_sms, cudaStream_t st) {
   if (ncol <= 0 || M <= 0 || K <= 0) return 0;
   const int tiles = ((ncol + BN - 1) / BN) * ((M + BM - 1) / BM);
   int ks = 1;
@@ -143,12 +141,12 @@ int launch_node_gemm(int M, int K, const float* A, const float* B, int64_t ldb, 
   int kchunk = ((K + ks - 1) / ks + BK - 1) / BK * BK;
   ks = (K + kchunk - 1) / kchunk;
   dim3 grid((ncol + BN - 1) / BN, (M + BM - 1) / BM, ks);
-  k_node_gemm<float><<<grid, NTH, 0, st>>>(M, K, kchunk, A, B, ldb, bidx, C, ldc, cidx, ncol, accumulate ? 1 : 0, sc,
-                                       ks > 1 ? ws : nullptr);
+  k_node_gemm<<<grid, NTH, 0, st>>>(M, K, kchunk, A, B, ldb, bidx, C, ldc, cidx, ncol, accumulate ? 1 : 0, sc,
+                                    ks > 1 ? ws : nullptr);
   if (ks > 1) {
     size_t n = (size_t)ncol * M;
     int g = (int)std::min<size_t>((n + 255) / 256, (size_t)num_sms * 8);
-    k_node_gemm_reduce<float><<<g, 256, 0, st>>>(M, ncol, ks, ws, C, ldc, cidx, accumulate ? 1 : 0, sc);
+    k_node_gemm_reduce<<<g, 256, 0, st>>>(M, ncol, ks, ws, C, ldc, cidx, accumulate ? 1 : 0, sc);
   }
   return ks > 1 ? 2 : 1;
 }

@@ -57,7 +57,7 @@ inline void launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t s
 template <typename T>
 struct P2PArgs {
   int nnodes = 0, ns = 0, nt = 0, nsurf = 0, nuc = 0;
-  const int *sbeg = nullptr, *scnt = nullptr, *tbeg = nullptr, *tcnt = nullptr, *depth = nullptr;
+  const int *sbeg = nullptr, *scnt = nullptr, *tbeg = nullptr, *tcnt = nullptr;
   const double *center = nullptr, *radius = nullptr;
   // sorted points, coordinates relative to their leaf centre
   const T *sx = nullptr, *sy = nullptr, *sz = nullptr, *snx = nullptr, *sny = nullptr, *snz = nullptr;

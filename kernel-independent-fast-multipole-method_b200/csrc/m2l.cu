@@ -1037,8 +1037,9 @@ __global__ void __launch_bounds__(NTHR) k_m2l_had_sweep(const Cpx<T>* __restrict
 // values per frequency, products of the differences above, formed in FP64 on
 // the host) is staged per tile of 16 frequencies; a warp carries two target
 // parents, one per half-warp, on the same 16 frequencies.
-constexpr int TZ_F = 16;          // frequencies per tile
-constexpr int TZ_ROWS = 26 * 28;  // transformed operator values per frequency (27 per direction, padded to 28)
+constexpr int TZ_F = 16;                      // frequencies per tile
+constexpr int TZ_THREADS = 512, TZ_NBUF = 2;  // one CTA per SM, the operator tile double-buffered
+constexpr int TZ_ROWS = 26 * 28;              // transformed operator values per frequency (27 per direction, padded to 28)
 
 // two consecutive transformed operator values of one frequency: layout
 // [dir][k/2][16][2] lets one 16-byte shared load (FP32) fetch both
@@ -1047,17 +1048,16 @@ struct __align__(4 * sizeof(T)) Cpx2 {
   Cpx<T> a, b;
 };
 
-template <typename T>
-__device__ __forceinline__ void cadd(Cpx<T>& r, const Cpx<T>& a, const Cpx<T>& b) {
+__device__ __forceinline__ void cadd(Cpx<float>& r, const Cpx<float>& a, const Cpx<float>& b) {
   r.re = a.re + b.re;
   r.im = a.im + b.im;
 }
 
-template <typename T, int NF, int SD, int TD>
-__device__ __forceinline__ void tz_tile(const Cpx<T>* __restrict__ Ts, const Cpx<T>* __restrict__ spectra,
+template <int NF, int SD, int TD>
+__device__ __forceinline__ void tz_tile(const Cpx<float>* __restrict__ Ts, const Cpx<float>* __restrict__ spectra,
                                         int* claim, int qend, int f, const int* __restrict__ qchd,
                                         const int* __restrict__ coll, const unsigned char* __restrict__ mask,
-                                        Cpx<T>* __restrict__ effval, int zero_node, int sc, int tc, bool acc_out) {
+                                        Cpx<float>* __restrict__ effval, int zero_node, int sc, int tc, bool acc_out) {
   constexpr int XS = SD * NF;  // source child stride
   const int lane = threadIdx.x & 31, hl = lane & 15, hw = lane >> 4;
   const int fl = min(f, NF - 1);  // lanes past NF load a valid spectrum and store nothing
@@ -1069,26 +1069,26 @@ __device__ __forceinline__ void tz_tile(const Cpx<T>* __restrict__ Ts, const Cpx
     const int q = q0 + hw;  // this half-warp's target parent
     const bool qv = q < qend;
     const int* cq = coll + (size_t)min(q, qend - 1) * 26;
-    Cpx<T> acc[27];
+    Cpx<float> acc[27];
 #pragma unroll
-    for (int k = 0; k < 27; k++) acc[k].re = acc[k].im = T(0);
-    Cpx<T> xa[8], xb[8];
+    for (int k = 0; k < 27; k++) acc[k].re = acc[k].im = 0.f;
+    Cpx<float> xa[8], xb[8];
     int nba, nbb;
-    auto load = [&](int dir, Cpx<T>* x, int& nb) {
+    auto load = [&](int dir, Cpx<float>* x, int& nb) {
       nb = qv ? cq[dir] : zero_node;
-      const Cpx<T>* X = spectra + ((size_t)nb * SD + sc) * NF + fl;
+      const Cpx<float>* X = spectra + ((size_t)nb * SD + sc) * NF + fl;
 #pragma unroll
       for (int j = 0; j < 8; j++) x[j] = X[j * XS];
     };
-    auto mult = [&](int dir, const Cpx<T>* x, int nb) {
+    auto mult = [&](int dir, const Cpx<float>* x, int nb) {
       if (!__any_sync(0xffffffffu, nb != zero_node)) return;
-      const Cpx2<T>* Td = reinterpret_cast<const Cpx2<T>*>(Ts) + (size_t)dir * 14 * TZ_F + hl;
-      Cpx2<T> tp;
+      const Cpx2<float>* Td = reinterpret_cast<const Cpx2<float>*>(Ts) + (size_t)dir * 14 * TZ_F + hl;
+      Cpx2<float> tp;
       // child j = (jx, jy, jz) bits (2, 1, 0); per axis the combinations
       // A = x(0) + x(1), B = x(1), C = x(0)
 #pragma unroll
       for (int kx = 0; kx < 3; kx++) {
-        Cpx<T> v[4];  // [jy][jz]
+        Cpx<float> v[4];  // [jy][jz]
 #pragma unroll
         for (int e = 0; e < 4; e++) {
           if (kx == 0) cadd(v[e], x[e], x[4 + e]);
@@ -1096,7 +1096,7 @@ __device__ __forceinline__ void tz_tile(const Cpx<T>* __restrict__ Ts, const Cpx
         }
 #pragma unroll
         for (int ky = 0; ky < 3; ky++) {
-          Cpx<T> w[2];  // [jz]
+          Cpx<float> w[2];  // [jz]
 #pragma unroll
           for (int e = 0; e < 2; e++) {
             if (ky == 0) cadd(w[e], v[e], v[2 + e]);
@@ -1104,12 +1104,12 @@ __device__ __forceinline__ void tz_tile(const Cpx<T>* __restrict__ Ts, const Cpx
           }
 #pragma unroll
           for (int kz = 0; kz < 3; kz++) {
-            Cpx<T> u;
+            Cpx<float> u;
             if (kz == 0) cadd(u, w[0], w[1]);
             else u = kz == 1 ? w[1] : w[0];
             const int k = (kx * 3 + ky) * 3 + kz;
             if ((k & 1) == 0) tp = Td[(k >> 1) * TZ_F];
-            const Cpx<T> t = (k & 1) ? tp.b : tp.a;
+            const Cpx<float> t = (k & 1) ? tp.b : tp.a;
             acc[k].re = fmt(-t.im, u.im, fmt(t.re, u.re, acc[k].re));
             acc[k].im = fmt(t.im, u.re, fmt(t.re, u.im, acc[k].im));
           }
@@ -1125,18 +1125,18 @@ __device__ __forceinline__ void tz_tile(const Cpx<T>* __restrict__ Ts, const Cpx
     }
     if (!qv || f >= NF) continue;
     // output combination per axis: y(0) = A + B, y(1) = A + C
-    Cpx<T> r[18];  // [kx][ky][iz]
+    Cpx<float> r[18];  // [kx][ky][iz]
 #pragma unroll
     for (int g = 0; g < 9; g++) {
       cadd(r[2 * g], acc[3 * g], acc[3 * g + 1]);
       cadd(r[2 * g + 1], acc[3 * g], acc[3 * g + 2]);
     }
-    Cpx<T> s4[12];  // [kx][iy][iz]
+    Cpx<float> s4[12];  // [kx][iy][iz]
 #pragma unroll
     for (int kx = 0; kx < 3; kx++)
 #pragma unroll
       for (int iz = 0; iz < 2; iz++) {
-        const Cpx<T> a0 = r[(kx * 3 + 0) * 2 + iz], b0 = r[(kx * 3 + 1) * 2 + iz], c0 = r[(kx * 3 + 2) * 2 + iz];
+        const Cpx<float> a0 = r[(kx * 3 + 0) * 2 + iz], b0 = r[(kx * 3 + 1) * 2 + iz], c0 = r[(kx * 3 + 2) * 2 + iz];
         cadd(s4[(kx * 2 + 0) * 2 + iz], a0, b0);
         cadd(s4[(kx * 2 + 1) * 2 + iz], a0, c0);
       }
@@ -1144,17 +1144,17 @@ __device__ __forceinline__ void tz_tile(const Cpx<T>* __restrict__ Ts, const Cpx
     const unsigned m = mask[q];
 #pragma unroll
     for (int e = 0; e < 4; e++) {  // (iy, iz)
-      Cpx<T> y[2];
+      Cpx<float> y[2];
       cadd(y[0], s4[0 * 4 + e], s4[1 * 4 + e]);
       cadd(y[1], s4[0 * 4 + e], s4[2 * 4 + e]);
 #pragma unroll
       for (int ix = 0; ix < 2; ix++) {
         const int i = ix * 4 + e;
         if (!((m >> i) & 1)) continue;
-        Cpx<T>* py = effval + ((size_t)(c0 + i) * TD + tc) * NF + f;
-        Cpx<T> v = y[ix];
+        Cpx<float>* py = effval + ((size_t)(c0 + i) * TD + tc) * NF + f;
+        Cpx<float> v = y[ix];
         if (acc_out) {
-          const Cpx<T> o = *py;
+          const Cpx<float> o = *py;
           v.re += o.re;
           v.im += o.im;
         }
@@ -1164,27 +1164,26 @@ __device__ __forceinline__ void tz_tile(const Cpx<T>* __restrict__ Ts, const Cpx
   }
 }
 
-template <typename T, int NF, int NTHR, int NBUF, int SD, int TD>
-__global__ void __launch_bounds__(NTHR) k_m2l_had_tz(const Cpx<T>* __restrict__ ttiles,
-                                                    const Cpx<T>* __restrict__ spectra, int nq,
+template <int NF, int SD, int TD>
+__global__ void __launch_bounds__(TZ_THREADS) k_m2l_had_tz(const Cpx<float>* __restrict__ ttiles,
+                                                    const Cpx<float>* __restrict__ spectra, int nq,
                                                     const int* __restrict__ qchd, const int* __restrict__ coll,
                                                     const unsigned char* __restrict__ mask,
-                                                    Cpx<T>* __restrict__ effval, int zero_node, int sc, int tc, int acc,
+                                                    Cpx<float>* __restrict__ effval, int zero_node, int sc, int tc, int acc,
                                                     int* __restrict__ status) {
   constexpr int TILE = TZ_ROWS * TZ_F;
-  constexpr unsigned TILE_BYTES = TILE * sizeof(Cpx<T>);
+  constexpr unsigned TILE_BYTES = TILE * sizeof(Cpx<float>);
   constexpr int FTILES = (NF + TZ_F - 1) / TZ_F;
-  constexpr int NW = NTHR / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cpx<T>* Tbuf = reinterpret_cast<Cpx<T>*>(smem_raw);  // NBUF x [26][27][16]
-  __shared__ __align__(8) unsigned long long bars[NBUF];
-  __shared__ int claim[NBUF], done_cnt[NBUF];
+  Cpx<float>* Tbuf = reinterpret_cast<Cpx<float>*>(smem_raw);  // TZ_NBUF x [26][14][16][2]
+  __shared__ __align__(8) unsigned long long bars[TZ_NBUF];
+  __shared__ int claim[TZ_NBUF], done_cnt[TZ_NBUF];
   const int lane = threadIdx.x & 31;
   const int per_cta = (nq + gridDim.x - 1) / gridDim.x;
   const int qbeg = blockIdx.x * per_cta;
   const int qend = min(nq, qbeg + per_cta);
   if (threadIdx.x == 0) {
-    for (int b = 0; b < NBUF; b++) {
+    for (int b = 0; b < TZ_NBUF; b++) {
       mbar_init(smem_addr(&bars[b]), 1);
       claim[b] = qbeg;
       done_cnt[b] = 0;
@@ -1201,10 +1200,10 @@ __global__ void __launch_bounds__(NTHR) k_m2l_had_tz(const Cpx<T>* __restrict__ 
       if (lane == 0) atomicOr(status, 1);
       return;
     }
-    tz_tile<T, NF, SD, TD>(Tbuf + (size_t)b * TILE, spectra, &claim[b], qend, ft * TZ_F + (lane & 15), qchd, coll,
+    tz_tile<NF, SD, TD>(Tbuf + (size_t)b * TILE, spectra, &claim[b], qend, ft * TZ_F + (lane & 15), qchd, coll,
                            mask, effval, zero_node, sc, tc, acc != 0);
     if (lane == 0) {
-      if (atomicAdd(&done_cnt[b], 1) == NW - 1) {  // the last warp out of tile ft
+      if (atomicAdd(&done_cnt[b], 1) == TZ_THREADS / 32 - 1) {  // the last warp out of tile ft
         done_cnt[b] = 0;
         claim[b] = qbeg;
         if (ft + 2 < FTILES)
@@ -1216,31 +1215,30 @@ __global__ void __launch_bounds__(NTHR) k_m2l_had_tz(const Cpx<T>* __restrict__ 
   }
 }
 
-template <typename T, int NF, int SD, int TD>
-void tz_launch(const T* ttiles, const T* spectra, int nq, const int* qchd, const int* coll, const unsigned char* mask,
-               T* effval, int zero_node, int* status, int num_sms, cudaStream_t st) {
-  constexpr int NTHR = 512, NBUF = 2;
-  const size_t smem = (size_t)NBUF * TZ_ROWS * TZ_F * sizeof(Cpx<T>);
-  auto kern = k_m2l_had_tz<T, NF, NTHR, NBUF, SD, TD>;
+template <int NF, int SD, int TD>
+void tz_launch(const float* ttiles, const float* spectra, int nq, const int* qchd, const int* coll, const unsigned char* mask,
+               float* effval, int zero_node, int* status, int num_sms, cudaStream_t st) {
+  const size_t smem = (size_t)TZ_NBUF * TZ_ROWS * TZ_F * sizeof(Cpx<float>);
+  auto kern = k_m2l_had_tz<NF, SD, TD>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int grid = std::max(1, std::min(num_sms, nq / 32));
   const size_t tiles = (size_t)((NF + TZ_F - 1) / TZ_F) * TZ_ROWS * TZ_F;  // Cpx per (t, s) table
   for (int t = 0; t < TD; t++)
     for (int s = 0; s < SD; s++)
-      kern<<<grid, NTHR, smem, st>>>(reinterpret_cast<const Cpx<T>*>(ttiles) + (size_t)(t * SD + s) * tiles,
-                                     reinterpret_cast<const Cpx<T>*>(spectra), nq, qchd, coll, mask,
-                                     reinterpret_cast<Cpx<T>*>(effval), zero_node, s, t, s > 0 ? 1 : 0, status);
+      kern<<<grid, TZ_THREADS, smem, st>>>(reinterpret_cast<const Cpx<float>*>(ttiles) + (size_t)(t * SD + s) * tiles,
+                                     reinterpret_cast<const Cpx<float>*>(spectra), nq, qchd, coll, mask,
+                                     reinterpret_cast<Cpx<float>*>(effval), zero_node, s, t, s > 0 ? 1 : 0, status);
 }
 
-template <typename T, int NF>
-void tz_dofs(int sd, int td, const T* ttiles, const T* spectra, int nq, const int* qchd, const int* coll,
-             const unsigned char* mask, T* effval, int zero_node, int* status, int num_sms, cudaStream_t st) {
+template <int NF>
+void tz_dofs(int sd, int td, const float* ttiles, const float* spectra, int nq, const int* qchd, const int* coll,
+             const unsigned char* mask, float* effval, int zero_node, int* status, int num_sms, cudaStream_t st) {
   if (sd == 1 && td == 1)
-    tz_launch<T, NF, 1, 1>(ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_launch<NF, 1, 1>(ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
   else if (sd == 4 && td == 3)
-    tz_launch<T, NF, 4, 3>(ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_launch<NF, 4, 3>(ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
   else if (sd == 3 && td == 3)
-    tz_launch<T, NF, 3, 3>(ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_launch<NF, 3, 3>(ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
 }
 
 template <typename T, int NF, int SD, int TD>
@@ -1302,11 +1300,11 @@ void launch_m2l_hadamard_tz(int nf, int sd, int td, const float* ttiles, const f
                             int num_sms, cudaStream_t st) {
   if (nq <= 0) return;
   if (nf == 668)
-    tz_dofs<float, 668>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_dofs<668>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
   else if (nf == 172)
-    tz_dofs<float, 172>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_dofs<172>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
   else if (nf == 1688)
-    tz_dofs<float, 1688>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
+    tz_dofs<1688>(sd, td, ttiles, spectra, nq, qchd, coll, mask, effval, zero_node, status, num_sms, st);
 }
 
 #define KIFMM_INST(T)                                                                                             \
