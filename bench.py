@@ -250,9 +250,9 @@ NF6 = 668  # stored (Hermitian-canonical) frequencies per spectrum at np=6: (11^
 NSURF6 = 6 ** 3 - 4 ** 3  # |UE| = |DC| at np=6
 # DRAM bytes (read + write) of one k_m2l_had_tc16 launch per spectrum node,
 # from an ncu capture of that kernel (dram__bytes_read.sum +
-# dram__bytes_write.sum) on the 1,048,576-point cloud of this workload,
+# dram__bytes_write.sum, profiles/hadamard_tc16_*) on the 1,048,576-point cloud of this workload,
 # scaled by the number of spectra of the workload timed here
-HAD_TRAFFIC_PER_SPECTRUM = 10338.0
+HAD_TRAFFIC_PER_SPECTRUM = 10348.0
 
 
 def roofline(phases, wc, hbm, bf16, sm_mhz, had_ms):

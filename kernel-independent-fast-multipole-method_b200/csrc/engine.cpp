@@ -90,7 +90,7 @@ std::shared_ptr<Tc16Images> tc16_images(const std::shared_ptr<const Operators>& 
   return p;
 }
 
-// The operator tables of the FP64 Hadamard, shared and freed in the same way (Navier np = 8: 207 MB).
+// The operator tables of the FP64 Hadamard, shared and freed in the same way (Navier np = 8: 171 MB).
 struct Had64Tables {
   double* t = nullptr;
   int device = 0;

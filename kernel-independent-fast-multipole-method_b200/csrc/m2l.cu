@@ -4,8 +4,8 @@
 //
 // The surface density of a node is a sparse n^3 grid, n = 2 np - 1 (np source
 // and np target points per axis have 2 np - 1 lags, so this is the smallest
-// cyclic size without wrap-around; the reference's 2 np holds 18 to 34 % more
-// frequencies): only the np^3 corner block holds data, and only on its boundary.  Instead of a general
+// cyclic size without wrap-around; the reference's 2 np holds 51, 30 and 22 %
+// more frequencies at np = 4, 6 and 8): only the np^3 corner block holds data, and only on its boundary.  Instead of a general
 // FFT library the transforms are pruned separable DFTs done in shared
 // memory, one CTA per node:
 //   forward : x pass (np^2 lines, np inputs -> np outputs), y pass, z pass

@@ -5,7 +5,7 @@
 //   surface grids      MatMgnt3d::splposcal, fmm3d/matmgnt3d.cpp:375-398
 //   UC2UE, DC2DE       pseudo-inverses, fmm3d/matmgnt3d.cpp:91-123,158-188
 //   UE2UC, DE2DC       child/parent matrices, fmm3d/matmgnt3d.cpp:125-156,190-221
-//   M2L spectra        FFT of the kernel sampled on the (2np)^3 grid,
+//   M2L spectra        DFT of the kernel sampled on the (2 np - 1)^3 grid,
 //                      fmm3d/matmgnt3d.cpp:296-361 (regposcal :400-420)
 //
 // The device passes use the pseudo-inverses in factored form (see Operators);
